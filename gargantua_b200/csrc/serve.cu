@@ -5,13 +5,13 @@
 // request, with one queue per metric: Schwarzschild rays and Kerr rays run
 // different integrators, so a warp works one queue at a time (half the
 // warps start on each, then take the other). Each warp steals chunks with
-// one atomic per chunk and keeps its 32 lanes busy: a lane whose ray ended
-// is refilled from the warp's chunk (ballot + popc ranks the idle lanes) as
-// soon as a quarter of the warp is idle, so long and short rays share warps
-// without the 8x8-tile tail of the per-request kernel. Ray state stays in
-// registers for the whole ray. Per-request counters are aggregated across
-// the lanes of a warp that finish together (match_any + reduce) before one
-// atomic per request. Rays over their drift budget after passing inside
+// one atomic per chunk and runs its rays to their ends, two neighbouring
+// Kerr rays to a lane (pairs.cuh); under the lane-refill schedule a lane
+// whose ray ended is refilled from the warp's chunk (ballot + popc ranks the
+// idle lanes) as soon as a quarter of the warp is idle, so long and short
+// rays share warps. Ray state stays in registers for the whole ray.
+// Per-request counters are aggregated across the lanes of a warp that finish
+// together (match_any + reduce) before one atomic per request. Rays over their drift budget after passing inside
 // r = 4 are queued for an FP64 re-integration kernel that runs after the
 // wave. The wave (counter reset, persistent kernel, FP64 pass) is captured
 // once per slot into a CUDA graph and replayed; only the wave's descriptors
@@ -37,7 +37,7 @@
 #include <thread>
 #include <vector>
 
-#include "lanes.cuh"
+#include "pairs.cuh"
 #include "runtime.h"
 
 namespace gg {
@@ -85,6 +85,7 @@ struct WaveArgs {
     uint32_t fp64_all;         // GG_FP64_ALL_FLAGGED
     uint32_t steps_per_round;  // RK4 steps between refill checks
     uint32_t refill_idle;      // refill once this many lanes of a warp are idle
+    float minus_zero;          // -0, a value the assembler does not know (pairs.cuh)
 };
 
 constexpr unsigned kFull = 0xffffffffu;
@@ -136,7 +137,9 @@ __device__ __forceinline__ void complete(const WaveArgs& a, uint32_t req, uint32
 
 template <int Kind> struct LaneOf;
 template <> struct LaneOf<0> { typedef SLane<float> type; };
-template <> struct LaneOf<1> { typedef KLane<float> type; };
+template <> struct LaneOf<1> { typedef KerrRays<float> type; };
+
+__device__ __forceinline__ uint32_t step_cap(const MarchUniforms& u) { return min(u.geodesic.stepCap, STEP_CAP_STILL); }
 
 template <int Kind>
 __device__ void serve_queue(const WaveArgs& a, uint32_t lane) {
@@ -146,7 +149,7 @@ __device__ void serve_queue(const WaveArgs& a, uint32_t lane) {
     const unsigned lower = (1u << lane) - 1u;
     typename LaneOf<Kind>::type L;
     bool active = false;
-    uint32_t req = 0, pixel = 0;
+    uint32_t req = 0, pixel = 0, taken = 0;  // taken: a Kerr ray's steps so far
     uint32_t cursor = 0, chunk_end = 0, chunk_req = 0;
     bool drained = false;
     for (uint32_t round = 0; round < kMaxRounds; ++round) {
@@ -189,7 +192,9 @@ __device__ void serve_queue(const WaveArgs& a, uint32_t lane) {
                         active = true;
                     }
                 } else {
-                    k_init(L, origin, dir, R.u);
+                    const KLane<float> l = kerr_launched(R.u, pixel);
+                    kerr_load(L, &l, &R.u.geodesic.stepMax);
+                    taken = 0;
                     active = true;
                 }
             }
@@ -215,8 +220,12 @@ __device__ void serve_queue(const WaveArgs& a, uint32_t lane) {
                         r = s_finish(L, R.u, t, a.blackbody);
                     }
                 } else {
-                    finished = k_step(L, R.u, R.emission, R.velocity, R.emission != 0);
-                    if (finished) r = k_finish(L, R.u, a.blackbody);
+                    const LaneView v{R.u.geodesic.stepFactor, R.u.geodesic.escapeRadius, a.minus_zero, R.emission != 0, &R.u, R.emission,
+                                     R.velocity};
+                    kerr_step(L, v, taken);
+                    if (++taken >= step_cap(R.u)) kerr_exhaust(L, taken);
+                    finished = !any_alive(L.sh);
+                    if (finished) r = kerr_finish(L, 0, R.u, a.blackbody);
                 }
                 budget = R.u.driftBudget;
                 if (finished) {
@@ -238,17 +247,15 @@ __device__ void serve_queue(const WaveArgs& a, uint32_t lane) {
 // thread-per-pixel image kernel; one warp-aggregated account per 32 rays.
 // The request's uniforms are copied to registers once per chunk, so the
 // step loop reads them as it would read kernel parameters.
-template <int Kind>
-__device__ void serve_chunks(const WaveArgs& a, uint32_t lane) {
-    const ServeChunk* chunks = Kind == 0 ? a.chunks0 : a.chunks1;
-    const uint32_t nchunks = a.header->chunk_count[Kind];
-    uint32_t* head = &a.header->heads[Kind];
+__device__ void serve_schwarzschild_chunks(const WaveArgs& a, uint32_t lane) {
+    const uint32_t nchunks = a.header->chunk_count[0];
+    uint32_t* head = &a.header->heads[0];
     for (uint32_t round = 0; round < kMaxRounds; ++round) {
         uint32_t c = 0;
         if (lane == 0) c = atomicAdd(head, 1u);
         c = __shfl_sync(kFull, c, 0);
         if (c >= nchunks) break;
-        const ServeChunk ch = chunks[c];
+        const ServeChunk ch = a.chunks0[c];
         const ServeRequest& R = a.requests[ch.request];
         const MarchUniforms u = R.u;
         const cudaTextureObject_t em = R.emission, vel = R.velocity;
@@ -261,24 +268,16 @@ __device__ void serve_chunks(const WaveArgs& a, uint32_t lane) {
                 const uint32_t w = u.resolution.x;
                 float3 dir = camera_direction(u, pixel % w, pixel / w);
                 float3 origin = to_f3(u.cameraPosition);
-                typename LaneOf<Kind>::type L;
-                if constexpr (Kind == 0) {
-                    float3 sky;
-                    SweepTables t{a.sphere_table, R.camera_table, R.sky_table};
-                    if (s_init(L, origin, dir, u, t, &sky)) {
-                        r = sky_only_result(sky, u, a.blackbody);
-                        write_result(R, pixel, r);
-                    } else {
-                        for (uint32_t s = 0; s <= STEP_CAP_STILL; ++s)
-                            if (s_step(L, u, em, vel, em != 0)) break;
-                        r = s_finish(L, u, t, a.blackbody);
-                        complete(a, ch.request, pixel, r);
-                    }
+                SLane<float> L;
+                float3 sky;
+                SweepTables t{a.sphere_table, R.camera_table, R.sky_table};
+                if (s_init(L, origin, dir, u, t, &sky)) {
+                    r = sky_only_result(sky, u, a.blackbody);
+                    write_result(R, pixel, r);
                 } else {
-                    k_init(L, origin, dir, u);
                     for (uint32_t s = 0; s <= STEP_CAP_STILL; ++s)
-                        if (k_step(L, u, em, vel, em != 0)) break;
-                    r = k_finish(L, u, a.blackbody);
+                        if (s_step(L, u, em, vel, em != 0)) break;
+                    r = s_finish(L, u, t, a.blackbody);
                     complete(a, ch.request, pixel, r);
                 }
             }
@@ -287,16 +286,91 @@ __device__ void serve_chunks(const WaveArgs& a, uint32_t lane) {
     }
 }
 
+// A chunk of Kerr rays (pairs.cuh) with R's rays in every lane, neighbouring
+// pixels beside each other: their rays take nearly the same number of steps,
+// so little is lost to a lane whose first ray ended. A warp's counters are
+// summed over its lanes once per 32 N rays: they all belong to one request.
+template <typename R>
+__device__ __forceinline__ void kerr_chunk(const WaveArgs& a, const ServeChunk& ch, const ServeRequest& q,
+                                           const WarpView& view, uint32_t lane) {
+    constexpr uint32_t N = Rays<R>::N;
+    const uint32_t cap = step_cap(q.u);
+    for (uint32_t base = 0; base < ch.count; base += 32u * N) {
+        const uint32_t first = base + N * lane;
+        KerrRays<R> p;
+        {
+            KLane<float> l[N];
+            float longest[N];
+#pragma unroll
+            for (uint32_t j = 0; j < N; ++j) {
+                // A lane past the chunk's end launches its last ray and drops it.
+                l[j] = kerr_launched(q.u, ch.first + min(first + j, ch.count - 1u));
+                longest[j] = first + j < ch.count ? q.u.geodesic.stepMax : 0.0f;
+            }
+            kerr_load(p, l, longest);
+        }
+        for (uint32_t step = 0; step < cap && any_alive(p.sh); ++step) kerr_step(p, view, step);
+        kerr_exhaust(p, cap);
+        uint32_t steps = 0, samples = 0, over = 0, exhausted = 0, captured = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < N; ++j) {
+            if (first + j >= ch.count) continue;
+            const PixelResult r = kerr_finish(p, (int)j, q.u, a.blackbody);
+            complete(a, ch.request, ch.first + first + j, r);
+            steps += r.steps;
+            samples += r.samples;
+            over += r.drift > q.u.driftBudget ? 1u : 0u;
+            exhausted += r.outcome == RayExhausted ? 1u : 0u;
+            captured += r.outcome == RayCaptured ? 1u : 0u;
+        }
+        steps = __reduce_add_sync(kFull, steps);
+        samples = __reduce_add_sync(kFull, samples);
+        over = __reduce_add_sync(kFull, over);
+        exhausted = __reduce_add_sync(kFull, exhausted);
+        captured = __reduce_add_sync(kFull, captured);
+        if (lane == 0) {
+            unsigned long long* st = q.stats;
+            if (steps) atomicAdd(st + 0, (unsigned long long)steps);
+            if (samples) atomicAdd(st + 1, (unsigned long long)samples);
+            atomicAdd(st + 3, (unsigned long long)min(32u * N, ch.count - base));
+            if (over) atomicAdd(st + 4, (unsigned long long)over);
+            if (exhausted) atomicAdd(st + 5, (unsigned long long)exhausted);
+            if (captured) atomicAdd(st + 6, (unsigned long long)captured);
+        }
+    }
+}
+
+// The chunk schedule for Kerr rays, with R's rays to a lane.
+template <typename R>
+__device__ void serve_kerr_chunks(const WaveArgs& a, uint32_t lane, GatherWords* words) {
+    const uint32_t nchunks = a.header->chunk_count[1];
+    uint32_t* head = &a.header->heads[1];
+    for (uint32_t round = 0; round < kMaxRounds; ++round) {
+        uint32_t c = 0;
+        if (lane == 0) c = atomicAdd(head, 1u);
+        c = __shfl_sync(kFull, c, 0);
+        if (c >= nchunks) break;
+        const ServeChunk ch = a.chunks1[c];
+        const ServeRequest& q = a.requests[ch.request];
+        __syncwarp();
+        if (lane == 0) *words = GatherWords{q.emission, q.velocity, q.u.volumeHalfExtent, q.u.opacityScale, q.u.redshift, 0u};
+        __syncwarp();
+        const WarpView view{q.u.geodesic.stepFactor, q.u.geodesic.escapeRadius, a.minus_zero, q.emission != 0, words};
+        kerr_chunk<R>(a, ch, q, view, lane);
+    }
+}
+
 // One persistent kernel per metric and schedule; a wave runs the two
-// metrics side by side. All four are held to 7 blocks per SM (at most 72
-// registers, with a few dozen bytes of spills): the step is bound by
-// instruction issue, and more warps per SM keep the issue slots fuller.
-// Measured on the mixed stream (64 requests, A/B on one box): 4 blocks per
-// SM 76.9 G ray-steps/s, 5 78.7, 6 79.6, 7 80.4, 8 78.1 (its spills grow to
-// 80 bytes); the compiler unbounded picks 119 registers, 4 blocks. Compiling
-// every schedule under the same bound keeps their arithmetic, and so their
-// pixels, identical.
+// metrics side by side. The kernels with one ray to a lane are held to 7
+// blocks per SM (at most 72 registers, with a few dozen bytes of spills):
+// their step is bound by instruction issue, and more warps per SM keep the
+// issue slots fuller (measured on the mixed stream with one ray to a lane
+// everywhere, 64 requests, A/B on one box: 4 blocks per SM 76.9 G
+// ray-steps/s, 5 78.7, 6 79.6, 7 80.4, 8 78.1). Two Kerr rays to a lane need
+// 126 registers: 4 blocks per SM, without spills (5, with 180 bytes of
+// them: 91.4 against 94.5 G ray-steps/s).
 constexpr int kServeBlocksPerSM = 7;
+constexpr int kKerrBlocksPerSM = 4;
 
 __global__ void __launch_bounds__(kServeThreads, kServeBlocksPerSM) serve_schwarzschild_kernel(WaveArgs a) {
     serve_queue<0>(a, threadIdx.x & 31u);
@@ -307,17 +381,34 @@ __global__ void __launch_bounds__(kServeThreads, kServeBlocksPerSM) serve_kerr_k
 }
 
 __global__ void __launch_bounds__(kServeThreads, kServeBlocksPerSM) serve_schwarzschild_chunks_kernel(WaveArgs a) {
-    serve_chunks<0>(a, threadIdx.x & 31u);
+    serve_schwarzschild_chunks(a, threadIdx.x & 31u);
 }
 
-__global__ void __launch_bounds__(kServeThreads, kServeBlocksPerSM) serve_kerr_chunks_kernel(WaveArgs a) {
-    serve_chunks<1>(a, threadIdx.x & 31u);
+__global__ void __launch_bounds__(kServeThreads, kKerrBlocksPerSM) serve_kerr_chunks_kernel(WaveArgs a) {
+    __shared__ GatherWords words[kServeThreads / 32];
+    serve_kerr_chunks<F2>(a, threadIdx.x & 31u, words + (threadIdx.x >> 5));
+}
+
+// One Kerr ray to a lane, for the waves that hold few (see form_wave).
+__global__ void __launch_bounds__(kServeThreads, kServeBlocksPerSM) serve_kerr_single_chunks_kernel(WaveArgs a) {
+    __shared__ GatherWords words[kServeThreads / 32];
+    serve_kerr_chunks<float>(a, threadIdx.x & 31u, words + (threadIdx.x >> 5));
 }
 
 // FP64 re-integration of the wave's flagged rays.
+constexpr uint32_t kReintegratePerWarp = 8;
+
 __global__ void __launch_bounds__(128) serve_reintegrate_kernel(WaveArgs a) {
     const uint32_t n = min(a.header->flagged_count, a.flagged_capacity);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    // Few rays to a warp: a warp's time is that of every path its lanes take,
+    // and the pass ends with its slowest ray (a lone 800x450 still's 222
+    // rays: 0.88 ms with 32 to a warp, 0.80 with 8, 0.74 with 1). 8 keep the
+    // instructions it takes from the waves beside it few.
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u), warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32u;
+    const uint32_t per = min(32u, max((n + warps - 1u) / warps, kReintegratePerWarp));
+    const uint32_t lane = threadIdx.x & 31u;
+    if (lane >= per) return;
+    for (uint32_t i = warp * per + lane; i < n; i += warps * per) {
         unsigned long long e = a.flagged[i];
         uint32_t req = (uint32_t)(e >> 32), pixel = (uint32_t)e;
         const ServeRequest& R = a.requests[req];
@@ -422,7 +513,8 @@ struct WaveSlot {
     cudaEvent_t fork = nullptr, join = nullptr;
     cudaEvent_t fp64_done = nullptr;
     cudaEvent_t start = nullptr, stop = nullptr;
-    cudaGraphExec_t graph = nullptr;
+    cudaGraphExec_t graph[2] = {nullptr, nullptr};  // with Kerr rays two to a lane, and one
+    bool kerr_single = false;                       // the wave being formed takes graph[1]
     char* device = nullptr;  // header, requests, chunks0, chunks1, flagged
     char* host = nullptr;    // pinned staging for the descriptors
     bool busy = false;
@@ -440,7 +532,7 @@ struct gg_server {
     uint32_t max_chunks = 0;
     uint32_t flagged_capacity = 0;
     uint64_t slot_bytes = 0;
-    int grid_s = 0, grid_k = 0;
+    int grid_s = 0, grid_k = 0, grid_k1 = 0;  // blocks of the Schwarzschild, Kerr and one-to-a-lane Kerr kernels
     cudaStream_t build = nullptr, copy = nullptr, plain = nullptr;
     // The server's own stream-ordered pool, keeping up to memory_bytes mapped
     // between requests so freeing one request's targets and allocating the
@@ -477,9 +569,10 @@ static uint64_t slot_offset_chunks1(const gg_server* s) { return slot_offset_chu
 static uint64_t slot_offset_flagged(const gg_server* s) { return slot_offset_chunks1(s) + (uint64_t)s->max_chunks * sizeof(ServeChunk); }
 
 // The wave graph: fork, the Schwarzschild and Kerr persistent kernels side
-// by side, join. The FP64 pass is launched outside the graph on its own
-// stream so it overlaps the next wave.
-static int capture_wave_graph(gg_server* s, WaveSlot& w) {
+// by side, join; a slot has one for each Kerr kernel of its schedule. The
+// FP64 pass is launched outside the graph on its own stream so it overlaps
+// the next wave.
+static int capture_wave_graph(gg_server* s, WaveSlot& w, bool single) {
     cudaGraph_t g = nullptr;
     GG_CUDA(cudaStreamBeginCapture(w.stream, cudaStreamCaptureModeThreadLocal), "wave capture");
     GG_CUDA(cudaEventRecord(w.fork, w.stream), "wave capture");
@@ -489,13 +582,14 @@ static int capture_wave_graph(gg_server* s, WaveSlot& w) {
         serve_kerr_kernel<<<s->grid_k, kServeThreads, 0, w.stream>>>(w.args);
     } else {
         serve_schwarzschild_chunks_kernel<<<s->grid_s, kServeThreads, 0, w.side>>>(w.args);
-        serve_kerr_chunks_kernel<<<s->grid_k, kServeThreads, 0, w.stream>>>(w.args);
+        if (single) serve_kerr_single_chunks_kernel<<<s->grid_k1, kServeThreads, 0, w.stream>>>(w.args);
+        else serve_kerr_chunks_kernel<<<s->grid_k, kServeThreads, 0, w.stream>>>(w.args);
     }
     GG_CUDA(cudaEventRecord(w.join, w.side), "wave capture");
     GG_CUDA(cudaStreamWaitEvent(w.stream, w.join, 0), "wave capture");
     cudaError_t e = cudaStreamEndCapture(w.stream, &g);
     GG_CUDA(e, "wave capture");
-    e = cudaGraphInstantiate(&w.graph, g, 0);
+    e = cudaGraphInstantiate(&w.graph[single ? 1 : 0], g, 0);
     cudaGraphDestroy(g);
     GG_CUDA(e, "wave graph instantiate");
     return GG_OK;
@@ -629,14 +723,28 @@ static bool form_wave(gg_server* s, WaveSlot& w) {
     ServeRequest* reqs = reinterpret_cast<ServeRequest*>(w.host + slot_offset_requests());
     ServeChunk* c0 = reinterpret_cast<ServeChunk*>(w.host + slot_offset_chunks0(s));
     ServeChunk* c1 = reinterpret_cast<ServeChunk*>(w.host + slot_offset_chunks1(s));
-    const uint32_t chunk = s->cfg.chunk_rays;
+    // Kerr rays go two to a lane, in chunks of at least the 64 that a warp
+    // takes at a time, unless the wave holds too few of them: a lane's two
+    // rays take longer than one, so with few rounds of chunks over the
+    // resident warps the last round, which waits for the longest rays, costs
+    // more than the pairs save. Lone stills in pairs against one ray to a
+    // lane: 230k rays +0.5 % (256 steps) and +10 % (4096 steps) of time, 518k
+    // -5 and +3 %, 705k -7 and +1 %, 921k -7 and -1 %, 2.1M -9 and -7 %. The
+    // line is at 4 rounds, 606k rays.
+    uint64_t kerr_rays = 0;
+    for (auto& r : cands)
+        if (r->u.spin > 0.0f) kerr_rays += r->rays - r->next_ray;
+    kerr_rays = std::min<uint64_t>(kerr_rays, s->cfg.wave_rays);
+    w.kerr_single = s->cfg.schedule == GG_SCHEDULE_CHUNKS &&
+                    kerr_rays < 4ull * 64u * (uint64_t)s->grid_k * (kServeThreads / 32);
+    const uint32_t chunks_of[2] = {s->cfg.chunk_rays, w.kerr_single ? s->cfg.chunk_rays : std::max(64u, s->cfg.chunk_rays)};
     uint64_t budget = s->cfg.wave_rays;
     w.members.clear();
     std::vector<uint32_t> local(cands.size(), UINT32_MAX);
     bool progress = true;
     while (budget > 0 && progress) {
         progress = false;
-        const uint64_t share = std::max<uint64_t>(chunk, budget / cands.size());
+        const uint64_t share = std::max<uint64_t>(chunks_of[1], budget / cands.size());
         for (size_t i = 0; i < cands.size() && budget > 0; ++i) {
             ServedRequest& r = *cands[i];
             if (r.next_ray >= r.rays) continue;
@@ -658,6 +766,7 @@ static bool form_wave(gg_server* s, WaveSlot& w) {
                 r.waves_pending += 1;
             }
             const int kind = r.u.spin > 0.0f ? 1 : 0;
+            const uint32_t chunk = chunks_of[kind];
             uint64_t take = std::min<uint64_t>({share, budget, (uint64_t)(r.rays - r.next_ray)});
             while (take > 0 && hdr->chunk_count[kind] < s->max_chunks) {
                 uint32_t n = (uint32_t)std::min<uint64_t>(chunk, take);
@@ -692,7 +801,7 @@ static int launch_wave(gg_server* s, WaveSlot& w) {
                                 hdr->chunk_count[1] * sizeof(ServeChunk), cudaMemcpyHostToDevice, w.stream),
                 "wave upload");
     GG_CUDA(cudaEventRecord(w.start, w.stream), "wave event");
-    GG_CUDA(cudaGraphLaunch(w.graph, w.stream), "wave launch");
+    GG_CUDA(cudaGraphLaunch(w.graph[w.kerr_single ? 1 : 0], w.stream), "wave launch");
     GG_CUDA(cudaEventRecord(w.stop, w.stream), "wave event");
     // FP64 pass after the wave, on its own stream: it overlaps the next wave.
     GG_CUDA(cudaStreamWaitEvent(w.fp64, w.stop, 0), "FP64 ordering");
@@ -952,6 +1061,10 @@ GG_API int gg_server_create(gg_context* ctx, const gg_volume* vol, const gg_serv
                 gg::kServeThreads, 0),
             "occupancy");
     s->grid_k = std::max(1, blocks) * ctx->sm_count;
+    GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, (const void*)gg::serve_kerr_single_chunks_kernel,
+                                                          gg::kServeThreads, 0),
+            "occupancy");
+    s->grid_k1 = std::max(1, blocks) * ctx->sm_count;
     {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
@@ -993,7 +1106,9 @@ GG_API int gg_server_create(gg_context* ctx, const gg_volume* vol, const gg_serv
         w.args.fp64_all = s->cfg.fp64_policy == GG_FP64_ALL_FLAGGED ? 1u : 0u;
         w.args.steps_per_round = s->cfg.steps_per_round;
         w.args.refill_idle = s->cfg.refill_idle;
-        GG_CHECK(gg::capture_wave_graph(s.get(), w));
+        w.args.minus_zero = -0.0f;
+        GG_CHECK(gg::capture_wave_graph(s.get(), w, false));
+        if (s->cfg.schedule == GG_SCHEDULE_CHUNKS) GG_CHECK(gg::capture_wave_graph(s.get(), w, true));
     }
     GG_CUDA(cudaStreamSynchronize(s->build), "server set-up");
     ctx->used += s->cfg.memory_bytes;  // reserved for admitted requests
@@ -1027,7 +1142,8 @@ void release_server_resources(gg_server* s) {
     for (auto& w : s->slots) {
         if (w.stream) cudaStreamSynchronize(w.stream);
         if (w.fp64) cudaStreamSynchronize(w.fp64);  // the FP64 pass reads the slot's flagged list
-        if (w.graph) cudaGraphExecDestroy(w.graph);
+        for (cudaGraphExec_t g : w.graph)
+            if (g) cudaGraphExecDestroy(g);
         if (w.device) gg::device_free(ctx, w.device, s->slot_bytes);
         if (w.host) cudaFreeHost(w.host);
         if (w.start) cudaEventDestroy(w.start);

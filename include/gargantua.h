@@ -503,7 +503,7 @@ typedef struct {
     int mode;                  /* gg_serve_mode */
     uint64_t memory_bytes;     /* device memory for admitted requests' targets; 0: a quarter of the budget left */
     uint32_t wave_rays;        /* rays packed into one persistent launch; 0: 4 Mi */
-    uint32_t chunk_rays;       /* rays per work-stealing chunk; 0: 32, one per lane of a warp */
+    uint32_t chunk_rays;       /* rays per work-stealing chunk; 0: 32, one per lane of a warp (Kerr rays: at least 64 where two share a lane) */
     uint32_t max_waves_in_flight; /* 0: 6; at most 8 */
     uint32_t fp64_policy;      /* gg_fp64_policy */
     uint32_t steps_per_round;  /* lane refill: RK4 steps a warp takes between refills of idle lanes; 0: 8 */

@@ -377,3 +377,29 @@ def test_bake_storage_counts_in_admission(world):
         server.submit(g.RequestSpec(320, 180, 256, 0.5, flags=g.types.REQUEST_BAKE))
     assert e.value.status == 8
     server.close()
+
+
+@pytest.mark.parametrize("width,height,cap,spin", [
+    (1101, 577, 40, 0.9),    # odd sizes, over the ray count from which two rays share a lane
+    (1101, 577, 1, 0.02),    # one step, barely spinning
+    (1280, 512, 300, 0.998),  # every lane full, captures beside a near-extremal horizon
+    (63, 3, 4096, 0.5),      # one ray to a lane: a last chunk of one lane less than full
+    (1, 1, 256, 0.9),
+])
+def test_kerr_rays_do_not_depend_on_their_lane(world, width, height, cap, spin):
+    """Kerr rays served two to a lane, one to a lane and by the lane-refill
+    schedule (always one) take the same steps and give the same bits."""
+    import gargantua_b200 as g
+
+    spec = g.RequestSpec(width, height, cap, spin, azimuth=0.8, elevation=0.15, distance=46.0)
+    got = []
+    for schedule in (g.types.SCHEDULE_CHUNKS, g.types.SCHEDULE_LANE_REFILL):
+        server = g.Server(world["ctx"], world["vol"], g.types.SERVE_BATCHED, schedule=schedule)
+        pixels, debug, res = server.wait(server.submit(spec, debug=True))
+        c = res.counters
+        got.append((pixels.view(np.uint16).copy(), debug.view(np.uint16).copy(), res.ray_steps, res.samples,
+                    res.fp64_rays, c.rays, c.overDriftBudget, c.exhausted, c.captured))
+        server.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+    assert got[0][5] == width * height and got[0][2] <= width * height * cap
