@@ -450,10 +450,8 @@ void bench(const Options& o) {
                 MarchUniforms ub = march_uniforms(o0, mw, mh, false, DRIFT_BUDGET_INTERACTIVE);
                 check(gg_tables_update(s.ctx, (float)o.distance, &ub));
                 ub.bakeSpacing = (float)(2.0 * VOLUME_HALF_EXTENT / s.size * BAKE_SPACING_VOXELS);  // BakePass.swift:50-52
-                auto bake_full = [&] {  // BAKE_FRAMES chunks of rows (BakePass.swift:55-84)
-                    const uint32_t rows = std::max(1u, mh / BAKE_FRAMES);
-                    for (uint32_t r = 0; r < mh; r += rows) check(gg_bake_rows(b, &ub, r, std::min(mh, r + rows)));
-                };
+                // encodeFullBake (BakePass.swift:55-84), its chunks of rows as one launch.
+                auto bake_full = [&] { check(gg_bake_rows(b, &ub, 0, mh)); };
                 fields.push_back(timing("bake_full", s.ctx, bake_full, 5));
                 uint32_t truncated = 0;
                 check(gg_bake_overflow(b, &truncated, 1));

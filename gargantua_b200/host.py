@@ -577,13 +577,12 @@ class Bake:
         check(lib().gg_bake_rows(self.handle, C.byref(u), row_begin, row_end))
 
     def bake_full(self, u: T.MarchUniforms, frames: int = 4):
-        """encodeFullBake: BAKE_FRAMES chunks of rows (BakePass.swift:55-84)."""
-        rows = max(self.height // frames, 1)
-        r = 0
-        while r < self.height:
-            n = min(rows, self.height - r)
-            self.bake_rows(u, r, r + n)
-            r += n
+        """encodeFullBake (BakePass.swift:55-84): every row. The reference
+        encodes BAKE_FRAMES chunks of rows, one a frame; issued together, as
+        here, they are one launch whatever `frames` is: at the end of each of
+        four the device waited for its longest rays (960x540: 774 us, one
+        launch 516 us)."""
+        self.bake_rows(u, 0, self.height)
 
     def overflow(self, reset: bool = False) -> int:
         c = C.c_uint32()
