@@ -494,7 +494,6 @@ struct ResolveArgs {
     const float4* __restrict__ blackbody;
     SplatUniforms u;
     double log_t_min, log_t_max;  // gg_log_d of the blackbody range, the same values on every device and host
-    uint32_t clear_mask;          // 0: the clear stores loaded & 0 (see resolve_kernel)
 };
 
 // Blackbody coordinate (Common.h:56-59) in double with the shared series
@@ -505,13 +504,15 @@ __device__ __forceinline__ float bb_coordinate_det(float temperature, double lo,
 }
 
 // resolveVolume (splat.metal:93-120) fused with the clear of the sums
-// (Volume.swift:34-43): each voxel's record is read once and written back
-// as zeros. The zeros are the loaded words ANDed with a mask of 0 passed at
-// launch, so each store waits for its own load: a store issued while the
-// read of its line is still in flight runs about 9x slower on B200 (a
-// 403 MB read-and-zero pass measured 0.73 TB/s that way, 6.3 TB/s with the
-// stores after the data). Rows come from the grid's y and z (no index
-// divisions).
+// (Volume.swift:34-43): each voxel's record is read once and, where it holds
+// anything, written back as zeros. It is bound by HBM: 24 bytes read and 16
+// written per voxel, and the clearing stores of the voxels that hold gas, a
+// tenth of a disk's cube (256^3 of the max preset: 204 us with every record
+// cleared, 131 this way; 128^3: 31 -> 24 us). The test on the loaded words
+// also makes each store wait for its own load: a store issued while the read
+// of its line is still in flight runs about 9x slower on B200 (a 403 MB
+// read-and-zero pass measured 0.73 TB/s that way, 6.3 TB/s with the stores
+// after the data). Rows come from the grid's y and z (no index divisions).
 
 // One voxel's record (E, E T, px, py, pz, mass) to its two texels.
 __device__ __forceinline__ void resolve_voxel(const ResolveArgs& a, uint32_t e, uint32_t et, uint32_t px, uint32_t py,
@@ -569,10 +570,7 @@ __global__ void __launch_bounds__(32 * kResolveRows) resolve_kernel(ResolveArgs 
     const uint64_t index = ((uint64_t)z * n + y) * n + x;
     uint2* rec = reinterpret_cast<uint2*>(a.sums + 6ull * index);
     uint2 r0 = rec[0], r1 = rec[1], r2 = rec[2];
-    const uint32_t m = a.clear_mask;
-    rec[0] = make_uint2(r0.x & m, r0.y & m);
-    rec[1] = make_uint2(r1.x & m, r1.y & m);
-    rec[2] = make_uint2(r2.x & m, r2.y & m);
+    if ((r0.x | r0.y | r1.x | r1.y | r2.x | r2.y) != 0u) rec[0] = rec[1] = rec[2] = make_uint2(0u, 0u);
     resolve_voxel(a, r0.x, r0.y, r1.x, r1.y, r2.x, r2.y, resolve_inverse_volume(a), x, y, z);
 }
 
@@ -908,7 +906,7 @@ GG_API int gg_splat_resolve(gg_volume* vol, const SplatUniforms* u, const gg_par
     std::lock_guard<std::recursive_mutex> lock(ctx->mu);
     GG_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
     ResolveArgs a{vol->sums, vol->emission_surf, vol->velocity_surf, ctx->blackbody, *u,
-                  gg_log_d((double)BLACKBODY_T_MIN), gg_log_d((double)BLACKBODY_T_MAX), 0u};
+                  gg_log_d((double)BLACKBODY_T_MIN), gg_log_d((double)BLACKBODY_T_MAX)};
     const uint32_t n = vol->size;
     resolve_kernel<<<dim3((n + 31u) / 32u, (n + kResolveRows - 1u) / kResolveRows, n), dim3(32, kResolveRows), 0,
                      ctx->stream>>>(a);

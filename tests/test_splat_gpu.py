@@ -213,3 +213,26 @@ def test_autotune_keeps_a_valid_shape_and_zeroed_sums(ctx, settled):
     rem, rmo, rma = O.deposit32(settled.read(), 64, frame=2, exact=True, seed=1)
     assert np.array_equal(em, rem) and np.array_equal(mo, rmo) and np.array_equal(ma, rma)
     vol.close()
+
+
+@pytest.mark.parametrize("size", [33, 40])
+def test_resolve_clears_records_of_any_one_word(ctx, size):
+    """A record is cleared whichever single word of it holds something."""
+    import gargantua_b200 as g
+
+    n3 = size ** 3
+    em, mo, ma = np.zeros(2 * n3, np.uint32), np.zeros(3 * n3, np.int32), np.zeros(n3, np.uint32)
+    voxels = np.random.default_rng(size).choice(n3, 60, replace=False)
+    for k, v in enumerate(voxels):
+        word = k % 6
+        if word < 2:
+            em[2 * v + word] = 1 + k
+        elif word < 5:
+            mo[3 * v + word - 2] = -1 - k
+        else:
+            ma[v] = 0x80000000
+    vol = g.Volume(ctx, size)
+    vol.write_sums(em, mo, ma)
+    vol.resolve()
+    assert not any(a.any() for a in vol.read_sums())
+    vol.close()
