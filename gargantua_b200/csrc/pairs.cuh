@@ -37,21 +37,6 @@ namespace gg {
 
 // ------------------------------------------------------------- arithmetic
 
-struct F2 {
-    unsigned long long v;
-};
-
-__device__ __forceinline__ F2 f2(float x, float y) {
-    F2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ float2 parts(F2 a) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
-    return r;
-}
-
 template <typename R> struct Rays;
 template <> struct Rays<float> {
     static constexpr int N = 1;
@@ -79,21 +64,6 @@ __device__ __forceinline__ float mad(float a, float b, float c) { return fmaf(a,
 __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float neg(float a) { return -a; }
-__device__ __forceinline__ F2 mad(F2 a, F2 b, F2 c) {
-    F2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return r;
-}
-__device__ __forceinline__ F2 mul(F2 a, F2 b) {
-    F2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
-}
-__device__ __forceinline__ F2 add(F2 a, F2 b) {
-    F2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
-}
 __device__ __forceinline__ F2 neg(F2 a) {
     const float2 p = parts(a);
     return f2(-p.x, -p.y);

@@ -275,8 +275,7 @@ __device__ void serve_schwarzschild_chunks(const WaveArgs& a, uint32_t lane) {
                     r = sky_only_result(sky, u, a.blackbody);
                     write_result(R, pixel, r);
                 } else {
-                    for (uint32_t s = 0; s <= STEP_CAP_STILL; ++s)
-                        if (s_step(L, u, em, vel, em != 0)) break;
+                    s_march<true>(L, u, em, vel, em != 0);
                     r = s_finish(L, u, t, a.blackbody);
                     complete(a, ch.request, pixel, r);
                 }

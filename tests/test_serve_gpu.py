@@ -403,3 +403,31 @@ def test_kerr_rays_do_not_depend_on_their_lane(world, width, height, cap, spin):
     for a, b in zip(*got):
         assert np.array_equal(a, b)
     assert got[0][5] == width * height and got[0][2] <= width * height * cap
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width,height,cap,distance", [
+    (333, 217, 4096, 46.0),  # onto the sphere and off it again
+    (96, 54, 1, 46.0),       # the one step the sphere's own loop takes
+    (95, 53, 256, 30.01),    # a camera just off it
+    (65, 37, 4096, 33.0),
+    (40, 40, 60, 200.0),     # out of steps on the way
+])
+def test_schwarzschild_rays_land_alike_in_both_loops(world, width, height, cap, distance):
+    """The chunk schedule marches the steps that cannot reach the sphere in a
+    loop without the landing; the lane-refill schedule takes every step with
+    it. Both take the same steps and give the same bits."""
+    import gargantua_b200 as g
+
+    spec = g.RequestSpec(width, height, cap, 0.0, azimuth=0.8, elevation=0.15, distance=distance)
+    got = []
+    for schedule in (g.types.SCHEDULE_CHUNKS, g.types.SCHEDULE_LANE_REFILL):
+        server = g.Server(world["ctx"], world["vol"], g.types.SERVE_BATCHED, schedule=schedule)
+        pixels, debug, res = server.wait(server.submit(spec, debug=True))
+        c = res.counters
+        got.append((pixels.view(np.uint16).copy(), debug.view(np.uint16).copy(), res.ray_steps, res.samples,
+                    res.fp64_rays, c.rays, c.overDriftBudget, c.exhausted, c.captured))
+        server.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+    assert got[0][5] == width * height
