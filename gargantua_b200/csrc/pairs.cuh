@@ -349,10 +349,9 @@ template <typename R> struct KerrRays {
 // A ray's drift and its pixel are out of line, compiled once for every kernel
 // and R, so that they round alike; the launch stays inline (out of line it
 // cost the served stream 3 %).
-__device__ __forceinline__ KLane<float> kerr_launched(const MarchUniforms& u, uint32_t pixel) {
+__device__ __forceinline__ KLane<float> kerr_launched(const MarchUniforms& u, uint2 pixel) {
     KLane<float> l;
-    const uint32_t w = u.resolution.x;
-    k_init(l, to_f3(u.cameraPosition), camera_direction(u, pixel % w, pixel / w), u);
+    k_init(l, to_f3(u.cameraPosition), camera_direction(u, pixel.x, pixel.y), u);
     return l;
 }
 __noinline__ __device__ float kerr_drift(const KLane<float>& l) { return k_drift(l); }

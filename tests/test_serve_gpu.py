@@ -431,3 +431,25 @@ def test_schwarzschild_rays_land_alike_in_both_loops(world, width, height, cap, 
     for a, b in zip(*got):
         assert np.array_equal(a, b)
     assert got[0][5] == width * height
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("spin", [0.0, 0.9])
+@pytest.mark.parametrize("width,height", [(1, 1), (7, 9), (8, 8), (9, 7), (16, 24), (65, 33), (3, 63), (101, 15)])
+def test_tiles_cover_images_of_any_size(world, width, height, spin):
+    """A served request's rays go through the image in tiles; each pixel gets
+    its own ray, as the per-pixel kernel marches it from the same uniforms
+    (the step counts' bounds are test_served_matches_plain_per_request's)."""
+    import gargantua_b200 as g
+
+    spec = g.RequestSpec(width, height, 4096, spin, azimuth=0.7, elevation=0.3, distance=50.0)
+    got = []
+    for mode in (g.types.SERVE_BATCHED, g.types.SERVE_SERIAL_PLAIN):
+        server = g.Server(world["ctx"], world["vol"], mode)
+        _, debug, res = server.wait(server.submit(spec, debug=True))
+        server.close()
+        assert res.counters.rays == width * height
+        got.append(debug.copy())
+    dsteps = np.abs(got[0][:, 1].astype(np.float32) - got[1][:, 1].astype(np.float32))
+    assert np.median(dsteps) <= 1.0, np.median(dsteps)
+    assert np.mean(dsteps <= 4.0) > 0.95, np.mean(dsteps <= 4.0)
