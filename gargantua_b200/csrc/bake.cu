@@ -37,7 +37,7 @@ struct BakeArgs {
 __global__ void __launch_bounds__(64) bake_kernel(BakeArgs a) {
     const MarchUniforms& u = a.p.u;
     const uint32_t gx = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t gy = blockIdx.y * blockDim.y + threadIdx.y;
+    const uint32_t gy = middle_out(blockIdx.y, gridDim.y) * blockDim.y + threadIdx.y;
     if (gy >= a.rows) return;
     const uint32_t px = u.tileOrigin.x + gx, py = u.tileOrigin.y + gy;
     if (px >= u.resolution.x || py >= u.resolution.y) return;

@@ -17,7 +17,7 @@ template <int Mode>
 __global__ void __launch_bounds__(256) march_image_kernel(MarchParams p) {
     constexpr bool Comp = Mode == GG_PRECISION_COMPENSATED || Mode == GG_PRECISION_RENORMALISED;
     const uint32_t gx = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t gy = blockIdx.y * blockDim.y + threadIdx.y;
+    const uint32_t gy = middle_out(blockIdx.y, gridDim.y) * blockDim.y + threadIdx.y;
     const uint32_t px = p.u.tileOrigin.x + gx, py = p.u.tileOrigin.y + gy;
     const bool inside = gx < p.target_width && gy < p.target_height;
     const bool active = inside && px < p.u.resolution.x && py < p.u.resolution.y;

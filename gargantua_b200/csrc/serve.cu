@@ -145,7 +145,7 @@ __device__ __forceinline__ void complete(const WaveArgs& a, uint32_t req, uint32
 // 256 steps 290 -> 240 us by both.
 __device__ __forceinline__ uint2 ray_pixel(const MarchUniforms& u, uint32_t index) {
     const uint32_t w = u.resolution.x, whole = u.resolution.y / 8u, k = index / (8u * w);
-    const uint32_t band = k < whole ? whole / 2u + ((k & 1u) ? 0u - (k + 1u) / 2u : k / 2u) : whole;
+    const uint32_t band = k < whole ? middle_out(k, whole) : whole;
     const uint32_t in_band = index - k * 8u * w, rows = min(8u, u.resolution.y - 8u * band);
     const uint32_t tile = min(in_band / (8u * rows), w / 8u);
     const uint32_t in_tile = in_band - tile * 8u * rows, columns = min(8u, w - 8u * tile);
