@@ -940,13 +940,15 @@ template <typename R> __device__ inline RayProbeResult k_probe_result(const KLan
 
 // One pixel through the lane path, run to completion: compensated FP32
 // (renormalised with Project), or the FP64 re-integration with R = double.
-template <typename R, bool Comp = true, bool Project = false>
+// Of one metric alone where the launch knows which (Metric 0: Schwarzschild,
+// 1: Kerr): a kernel of both takes the registers of the hungrier.
+template <typename R, bool Comp = true, bool Project = false, int Metric = -1>
 __device__ inline PixelResult shade_pixel_lane(const MarchParams& p, uint32_t px, uint32_t py) {
     const MarchUniforms& u = p.u;
     const bool gather = p.emission != 0;
     float3 dir = camera_direction(u, px, py);
     float3 origin = to_f3(u.cameraPosition);
-    if (u.spin > 0.0f) {
+    if (Metric == 1 || (Metric < 0 && u.spin > 0.0f)) {
         KLane<R> l;
         k_init(l, origin, dir, u);
         for (uint32_t k = 0; k <= STEP_CAP_STILL; ++k)
@@ -963,21 +965,6 @@ __device__ inline PixelResult shade_pixel_lane(const MarchParams& p, uint32_t px
             if (s_step<R, Comp, Project>(l, u, p.emission, p.velocity, gather)) break;
     }
     return s_finish(l, u, p.tables, p.blackbody);
-}
-
-__device__ inline PixelResult shade_pixel_compensated(const MarchParams& p, uint32_t px, uint32_t py) {
-    return shade_pixel_lane<float, true>(p, px, py);
-}
-
-// Compensated FP32 with the Hamiltonian-constraint renormalisation after
-// every step.
-__device__ inline PixelResult shade_pixel_renormalised(const MarchParams& p, uint32_t px, uint32_t py) {
-    return shade_pixel_lane<float, true, true>(p, px, py);
-}
-
-// The plain FP32 march: the same lane code with direct adds.
-__device__ inline PixelResult shade_pixel_plain(const MarchParams& p, uint32_t px, uint32_t py) {
-    return shade_pixel_lane<float, false>(p, px, py);
 }
 
 }  // namespace gg

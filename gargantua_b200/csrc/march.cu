@@ -12,8 +12,9 @@
 
 namespace gg {
 
-// Mode: GG_PRECISION_PLAIN, _COMPENSATED, _PLAIN_AS_WRITTEN or _RENORMALISED.
-template <int Mode>
+// Mode: GG_PRECISION_PLAIN, _COMPENSATED, _PLAIN_AS_WRITTEN or _RENORMALISED;
+// Metric: 1 for Kerr, 0 for Schwarzschild, -1 for either.
+template <int Mode, int Metric>
 __global__ void __launch_bounds__(256) march_image_kernel(MarchParams p) {
     constexpr bool Comp = Mode == GG_PRECISION_COMPENSATED || Mode == GG_PRECISION_RENORMALISED;
     const uint32_t gx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -24,10 +25,8 @@ __global__ void __launch_bounds__(256) march_image_kernel(MarchParams p) {
     PixelResult r{};
     r.outcome = RayEscaped;
     if (active) {
-        if constexpr (Mode == GG_PRECISION_COMPENSATED) r = shade_pixel_compensated(p, px, py);
-        else if constexpr (Mode == GG_PRECISION_RENORMALISED) r = shade_pixel_renormalised(p, px, py);
-        else if constexpr (Mode == GG_PRECISION_PLAIN) r = shade_pixel_plain(p, px, py);
-        else r = shade_pixel<float, false>(p, px, py);
+        if constexpr (Mode == GG_PRECISION_PLAIN_AS_WRITTEN) r = shade_pixel<float, false>(p, px, py);
+        else r = shade_pixel_lane<float, Comp, Mode == GG_PRECISION_RENORMALISED, Metric>(p, px, py);
         const uint32_t local = gy * p.target_width + gx;
         write_pixel(p, local, r);
         if (Comp && p.flagged && needs_fp64(p.u, r, p.fp64_all != 0u)) {
@@ -219,24 +218,27 @@ MarchParams make_params(gg_context* ctx, const gg_volume* vol, const MarchUnifor
     return p;
 }
 
+template <int Mode> static int launch_image(const MarchParams& p, cudaStream_t stream, const char* what) {
+    const dim3 block(p.block_w, p.block_h);
+    const dim3 grid((p.target_width + block.x - 1) / block.x, (p.target_height + block.y - 1) / block.y);
+    if constexpr (Mode == GG_PRECISION_PLAIN_AS_WRITTEN) march_image_kernel<Mode, -1><<<grid, block, 0, stream>>>(p);
+    else if (p.u.spin > 0.0f) march_image_kernel<Mode, 1><<<grid, block, 0, stream>>>(p);
+    else march_image_kernel<Mode, 0><<<grid, block, 0, stream>>>(p);
+    return launch_status(what);
+}
+
 // The compensated image march and its FP64 pass, given a parameter block
 // whose flagged list and counter are already set (p.flagged, p.flagged_count
 // zeroed by the caller, p.flagged_capacity entries).
 int launch_compensated_image(const MarchParams& p, cudaStream_t stream, int sm_count) {
-    dim3 block(p.block_w, p.block_h);
-    dim3 grid((p.target_width + block.x - 1) / block.x, (p.target_height + block.y - 1) / block.y);
-    march_image_kernel<GG_PRECISION_COMPENSATED><<<grid, block, 0, stream>>>(p);
-    GG_CHECK(launch_status("compensated march"));
+    GG_CHECK(launch_image<GG_PRECISION_COMPENSATED>(p, stream, "compensated march"));
     reintegrate_kernel<<<sm_count, 128, 0, stream>>>(p);
     return launch_status("FP64 re-integration");
 }
 
 int launch_plain_image(const MarchParams& p, cudaStream_t stream, bool as_written) {
-    dim3 block(p.block_w, p.block_h);
-    dim3 grid((p.target_width + block.x - 1) / block.x, (p.target_height + block.y - 1) / block.y);
-    if (as_written) march_image_kernel<GG_PRECISION_PLAIN_AS_WRITTEN><<<grid, block, 0, stream>>>(p);
-    else march_image_kernel<GG_PRECISION_PLAIN><<<grid, block, 0, stream>>>(p);
-    return launch_status("plain march");
+    if (as_written) return launch_image<GG_PRECISION_PLAIN_AS_WRITTEN>(p, stream, "plain march");
+    return launch_image<GG_PRECISION_PLAIN>(p, stream, "plain march");
 }
 
 static bool known_precision(int precision) {
@@ -388,19 +390,14 @@ GG_API int gg_march(gg_context* ctx, const gg_volume* vol, const MarchUniforms* 
         p.flagged_capacity = (uint32_t)entries;
         GG_CUDA(cudaMemsetAsync(ctx->flagged, 0, 4u, ctx->stream), "re-integration list reset");
     }
-    dim3 block(p.block_w, p.block_h);
-    dim3 grid((targets->width + block.x - 1) / block.x, (targets->height + block.y - 1) / block.y);
     if (comp) {
         if (precision == GG_PRECISION_RENORMALISED)
-            march_image_kernel<GG_PRECISION_RENORMALISED><<<grid, block, 0, ctx->stream>>>(p);
+            GG_CHECK(gg::launch_image<GG_PRECISION_RENORMALISED>(p, ctx->stream, "march"));
         else
-            march_image_kernel<GG_PRECISION_COMPENSATED><<<grid, block, 0, ctx->stream>>>(p);
-        GG_CHECK(gg::launch_status("march"));
+            GG_CHECK(gg::launch_image<GG_PRECISION_COMPENSATED>(p, ctx->stream, "march"));
         reintegrate_kernel<<<ctx->sm_count, 128, 0, ctx->stream>>>(p);
-    } else if (precision == GG_PRECISION_PLAIN) {
-        march_image_kernel<GG_PRECISION_PLAIN><<<grid, block, 0, ctx->stream>>>(p);
     } else {
-        march_image_kernel<GG_PRECISION_PLAIN_AS_WRITTEN><<<grid, block, 0, ctx->stream>>>(p);
+        GG_CHECK(gg::launch_plain_image(p, ctx->stream, precision == GG_PRECISION_PLAIN_AS_WRITTEN));
     }
     GG_CHECK(gg::launch_status("march"));
     if (counters) {
