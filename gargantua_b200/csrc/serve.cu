@@ -69,7 +69,8 @@ struct WaveHeader {
     uint32_t heads[2];
     uint32_t flagged_count;
     uint32_t request_count;
-    uint32_t pad[10];
+    uint32_t spare_blocks;  // of a Kerr kernel, that leave their places to another wave's FP64 pass
+    uint32_t pad[9];
 };
 static_assert(sizeof(WaveHeader) == 64, "WaveHeader");
 
@@ -404,17 +405,20 @@ __global__ void __launch_bounds__(kServeThreads, kServeBlocksPerSM) serve_schwar
 
 __global__ void __launch_bounds__(kServeThreads, kKerrBlocksPerSM) serve_kerr_chunks_kernel(WaveArgs a) {
     __shared__ GatherWords words[kServeThreads / 32];
+    if (blockIdx.x < a.header->spare_blocks) return;
     serve_kerr_chunks<F2>(a, threadIdx.x & 31u, words + (threadIdx.x >> 5));
 }
 
 // One Kerr ray to a lane, for the waves that hold few (see form_wave).
 __global__ void __launch_bounds__(kServeThreads, kServeBlocksPerSM) serve_kerr_single_chunks_kernel(WaveArgs a) {
     __shared__ GatherWords words[kServeThreads / 32];
+    if (blockIdx.x < a.header->spare_blocks) return;
     serve_kerr_chunks<float>(a, threadIdx.x & 31u, words + (threadIdx.x >> 5));
 }
 
 // FP64 re-integration of the wave's flagged rays.
 constexpr uint32_t kReintegratePerWarp = 8;
+constexpr uint32_t kSpareBlocks = 40;  // the FP64 pass of a 1920x1080 still: 1280 rays, 8 to a warp
 
 __global__ void __launch_bounds__(128) serve_reintegrate_kernel(WaveArgs a) {
     const uint32_t n = min(a.header->flagged_count, a.flagged_capacity);
@@ -565,6 +569,7 @@ struct gg_server {
     std::map<uint64_t, std::shared_ptr<gg::ServedRequest>> all;
     uint64_t next_ticket = 1;
     uint64_t memory_used = 0;
+    bool parted = false;  // the last wave formed was the first part of two (form_wave)
     bool stop = false;
     int fatal = GG_OK;
     std::string fatal_sentence;
@@ -756,7 +761,27 @@ static bool form_wave(gg_server* s, WaveSlot& w) {
     w.kerr_single = s->cfg.schedule == GG_SCHEDULE_CHUNKS &&
                     kerr_rays < 4ull * 64u * (uint64_t)s->grid_k * (kServeThreads / 32);
     const uint32_t chunks_of[2] = {s->cfg.chunk_rays, w.kerr_single ? s->cfg.chunk_rays : std::max(64u, s->cfg.chunk_rays)};
+    // Kerr rays that would make one last wave, with nothing else under way,
+    // make two: the rays flagged for FP64 pass close to the hole, so they are
+    // among the first two fifths (ray_pixel), and that part's FP64 pass, a
+    // millisecond of latency, runs beside the rest, which leaves it the places
+    // of kSpareBlocks blocks. Lone stills: 640x360 1380 -> 1190 us (256 steps)
+    // and 2210 -> 2120 (4096), 960x540 2260 -> 2080 and 3100 -> 2630,
+    // 1280x720 7080 -> 5970 (4096), 1920x1080 7080 -> 6230. The line is at one
+    // round of rays: below it the wave's end is that of its longest rays, and
+    // two waves end 1 to 2 % later.
     uint64_t budget = s->cfg.wave_rays;
+    const bool busy = std::any_of(s->slots.begin(), s->slots.end(), [](const WaveSlot& o) { return o.busy; });
+    if (s->parted && busy) {
+        hdr->spare_blocks = kSpareBlocks;
+        s->parted = false;
+    } else {
+        uint64_t left = 0;
+        for (auto& r : cands) left += r->rays - r->next_ray;
+        s->parted = !busy && s->slots.size() > 1 && s->cfg.schedule == GG_SCHEDULE_CHUNKS && left <= budget &&
+                    kerr_rays >= (uint64_t)s->grid_k1 * kServeThreads;
+        if (s->parted) budget = left * 2u / 5u & ~63ull;
+    }
     w.members.clear();
     std::vector<uint32_t> local(cands.size(), UINT32_MAX);
     bool progress = true;

@@ -453,3 +453,29 @@ def test_tiles_cover_images_of_any_size(world, width, height, spin):
     dsteps = np.abs(got[0][:, 1].astype(np.float32) - got[1][:, 1].astype(np.float32))
     assert np.median(dsteps) <= 1.0, np.median(dsteps)
     assert np.mean(dsteps <= 4.0) > 0.95, np.mean(dsteps <= 4.0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width,height,cap,spin", [
+    (487, 301, 256, 0.9),   # just over the rays from which a lone Kerr request makes two waves, one ray to a lane
+    (1203, 797, 60, 0.5),   # two rays to a lane
+    (640, 360, 4096, 0.998),
+])
+def test_a_request_in_two_waves_is_the_same(world, width, height, cap, spin):
+    """A lone Kerr request is marched in two waves where two may be in flight,
+    in one where only one may; the pixels and counters are the same."""
+    import gargantua_b200 as g
+
+    spec = g.RequestSpec(width, height, cap, spin, azimuth=0.8, elevation=0.3, distance=48.0)
+    got = []
+    for in_flight in (0, 1):
+        server = g.Server(world["ctx"], world["vol"], g.types.SERVE_BATCHED, max_waves_in_flight=in_flight)
+        pixels, debug, res = server.wait(server.submit(spec, debug=True))
+        waves = server.totals()["launches"] // 3
+        c = res.counters
+        got.append((pixels.view(np.uint16).copy(), debug.view(np.uint16).copy(), res.ray_steps, res.samples,
+                    res.fp64_rays, c.rays, c.overDriftBudget, c.exhausted, c.captured))
+        server.close()
+        assert waves == (2 if in_flight == 0 else 1)
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
