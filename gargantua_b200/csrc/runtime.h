@@ -149,8 +149,7 @@ struct gg_volume {
     uint64_t bytes = 0;
     // Splat shape per deposit mode ([0] stochastic, [1] exact): brick edge B
     // (0: direct global atomics) and particles per deposit work item.
-    uint32_t brick_edge[2] = {0u, 8u};    // [stochastic, exact]; set per size by gg_volume_create,
-                                          // chunk 0 of an edge: both by the number of particles
+    uint32_t brick_edge[2] = {0u, 8u};    // [stochastic, exact]; set per size by gg_volume_create
     uint32_t brick_chunk[2] = {0u, 1024u};
     void* brick_scratch = nullptr;  // counts, cursor, offsets, items, sorted slots, keys
     uint64_t brick_scratch_capacity = 0;

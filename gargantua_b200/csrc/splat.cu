@@ -758,14 +758,16 @@ GG_API int gg_volume_create(gg_context* ctx, uint32_t size, gg_volume** out) {
     gg_volume* vol = new gg_volume();
     vol->ctx = ctx;
     vol->size = size;
-    // Default shapes: the stochastic deposit (one corner per particle) is
-    // fastest with direct global atomics at every size; the exact one in 8^3
-    // bricks below 96^3 and by the number of particles from there
-    // (exact_shape).
+    // Default shapes, from timing the shapes on the presets' settled disks
+    // (250k/96^3, 1M/128^3, 4M/256^3, uniform and concentrated): the
+    // stochastic deposit (one corner per particle) is fastest with direct
+    // global atomics at every size; the exact one with 16^3 bricks from 96^3
+    // up (41, 73 and 230 us against 45, 83 and 620 us with 8^3 bricks), in
+    // chunks of 4096, 8192 and 16384 particles, and with 8^3 bricks below.
     vol->brick_edge[0] = 0u;
     vol->brick_chunk[0] = 0u;
     vol->brick_edge[1] = size >= 96u ? 16u : 8u;
-    vol->brick_chunk[1] = size >= 96u ? 0u : 1024u;
+    vol->brick_chunk[1] = size > 128u ? 16384u : size > 96u ? 8192u : size >= 96u ? 4096u : 1024u;
     int s = gg::device_alloc(ctx, sums_bytes, (void**)&vol->sums, "volume sums");
     if (s == GG_OK) s = gg::cuda_status(cudaMemsetAsync(vol->sums, 0, sums_bytes, ctx->stream), "volume clear");
     cudaChannelFormatDesc desc = cudaCreateChannelDescHalf4();
@@ -830,33 +832,6 @@ GG_API void gg_volume_destroy(gg_volume* vol) {
     delete vol;
 }
 
-// The exact deposit's shape for a number of particles, where none was set.
-// Up to 65536 particles, direct atomics: the bricks' four launches and a
-// block's zeroed tile take 27 to 40 us however few there are (50k particles:
-// 28, 23 and 22 us against 33, 30 and 40 into 96^3, 128^3 and 256^3; 100k: 46,
-// 36 and 35 against 28, 31 and 42). Above, 16^3 bricks in chunks that make
-// two thirds of a round of the deposit's blocks, one per SM, and from 800k
-// particles on five thirds: more rounds spread the bricks' unequal chunks
-// better, fewer flush less, and a little over one round is worst (200k into
-// 96^3: 32 us, 39 in chunks of 4096; 1M into 128^3: 66, 68 of 8192; 1.5M into
-// 96^3: 83, 87 of 4096; 3M into 128^3: 145, 151 of 8192). Beyond 128^3 the
-// bricks alone make more than a round until some 1.25M particles fill them:
-// the largest chunk (400k into 192^3: 46 us, 48 by the rounds).
-static void exact_shape(const gg_context* ctx, uint32_t size, uint32_t count, uint32_t* edge, uint32_t* chunk) {
-    constexpr uint32_t kSmallest = 1024u, kLargest = 16384u;
-    if (count <= 65536u) {
-        *edge = 0u;
-        *chunk = 0u;
-        return;
-    }
-    const uint64_t rounds3 = count < 800'000u ? 2u : 5u;
-    const uint64_t by_rounds = 3ull * count / (rounds3 * (uint64_t)ctx->sm_count);
-    *edge = 16u;
-    *chunk = size > 128u && count < 1'250'000u
-                 ? kLargest
-                 : (uint32_t)std::min<uint64_t>(std::max<uint64_t>(by_rounds, kSmallest), kLargest);
-}
-
 GG_API int gg_splat_bin(gg_particles* ps, gg_volume* vol, const SplatUniforms* u) {
     if (!ps) return gg::fail(GG_ERR_INVALID_ARGUMENT, "gg_splat_bin needs a particle system.");
     GG_CHECK(check_splat(ps, vol, u, "gg_splat_bin"));
@@ -864,9 +839,7 @@ GG_API int gg_splat_bin(gg_particles* ps, gg_volume* vol, const SplatUniforms* u
     std::lock_guard<std::recursive_mutex> lock(ctx->mu);
     GG_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
     const int mode = u->exactDeposit ? 1 : 0;
-    uint32_t edge = vol->brick_edge[mode], chunk = vol->brick_chunk[mode];
-    if (edge != 0u && chunk == 0u) exact_shape(ctx, vol->size, ps->count, &edge, &chunk);
-    return splat_bin_shaped(ps, vol, u, edge, chunk);
+    return splat_bin_shaped(ps, vol, u, vol->brick_edge[mode], vol->brick_chunk[mode]);
 }
 
 GG_API int gg_volume_splat_shape(gg_volume* vol, int exact, uint32_t brick_edge, uint32_t chunk) {

@@ -236,25 +236,3 @@ def test_resolve_clears_records_of_any_one_word(ctx, size):
     vol.resolve()
     assert not any(a.any() for a in vol.read_sums())
     vol.close()
-
-
-@pytest.mark.parametrize("size,count", [(96, 65_536), (96, 65_537), (129, 70_001), (128, 799_999), (128, 800_000),
-                                        (192, 1_249_999), (192, 1_250_000)])
-def test_default_exact_shapes_give_the_direct_sums(ctx, size, count):
-    """The shape chosen by the number of particles, at each edge of its rule,
-    against direct atomics: the same sums bit for bit."""
-    import gargantua_b200 as g
-
-    ps = g.Particles(ctx, count, seed=5)
-    ps.advance(20, seed_first=True)
-    got = []
-    for direct in (False, True):
-        vol = g.Volume(ctx, size)
-        if direct:
-            vol.set_shape(True, 0)
-        vol.bin(ps, True)
-        got.append(vol.read_sums())
-        vol.close()
-    ps.close()
-    for a, b in zip(*got):
-        assert a.any() and np.array_equal(a, b)
