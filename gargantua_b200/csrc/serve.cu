@@ -569,6 +569,7 @@ struct gg_server {
     std::map<uint64_t, std::shared_ptr<gg::ServedRequest>> all;
     uint64_t next_ticket = 1;
     uint64_t memory_used = 0;
+    bool kerr_single = false;  // the last wave formed has one Kerr ray to a lane
     bool parted = false;  // the last wave formed was the first part of two (form_wave)
     bool stop = false;
     int fatal = GG_OK;
@@ -750,16 +751,20 @@ static bool form_wave(gg_server* s, WaveSlot& w) {
     // takes at a time, unless the wave holds too few of them: a lane's two
     // rays take longer than one, so with few rounds of chunks over the
     // resident warps the last round, which waits for the longest rays, costs
-    // more than the pairs save. Lone stills in pairs against one ray to a
-    // lane: 230k rays +0.5 % (256 steps) and +10 % (4096 steps) of time, 518k
-    // -5 and +3 %, 705k -7 and +1 %, 921k -7 and -1 %, 2.1M -9 and -7 %. The
-    // line is at 4 rounds, 606k rays.
+    // more than the pairs save. Lone stills, one ray to a lane against pairs:
+    // 230k rays 1180 us, 1280 (256 steps) and 2110, 2430 (4096); 360k 1515,
+    // 1400 and 2240, 2410; 518k 2050, 1745 and 2680, 2660; 682k 2406, 2190
+    // and 3150, 2910. The line is at 3 rounds, 455k rays; the second part of
+    // two waves stays in pairs if the first was.
     uint64_t kerr_rays = 0;
     for (auto& r : cands)
         if (r->u.spin > 0.0f) kerr_rays += r->rays - r->next_ray;
     kerr_rays = std::min<uint64_t>(kerr_rays, s->cfg.wave_rays);
-    w.kerr_single = s->cfg.schedule == GG_SCHEDULE_CHUNKS &&
-                    kerr_rays < 4ull * 64u * (uint64_t)s->grid_k * (kServeThreads / 32);
+    const bool busy = std::any_of(s->slots.begin(), s->slots.end(), [](const WaveSlot& o) { return o.busy; });
+    const bool second = s->parted && busy;
+    s->kerr_single = s->cfg.schedule == GG_SCHEDULE_CHUNKS && !(second && !s->kerr_single) &&
+                     kerr_rays < 3ull * 64u * (uint64_t)s->grid_k * (kServeThreads / 32);
+    w.kerr_single = s->kerr_single;
     const uint32_t chunks_of[2] = {s->cfg.chunk_rays, w.kerr_single ? s->cfg.chunk_rays : std::max(64u, s->cfg.chunk_rays)};
     // Kerr rays that would make one last wave, with nothing else under way,
     // make two: the rays flagged for FP64 pass close to the hole, so they are
@@ -771,8 +776,7 @@ static bool form_wave(gg_server* s, WaveSlot& w) {
     // round of rays: below it the wave's end is that of its longest rays, and
     // two waves end 1 to 2 % later.
     uint64_t budget = s->cfg.wave_rays;
-    const bool busy = std::any_of(s->slots.begin(), s->slots.end(), [](const WaveSlot& o) { return o.busy; });
-    if (s->parted && busy) {
+    if (second) {
         hdr->spare_blocks = kSpareBlocks;
         s->parted = false;
     } else {
