@@ -494,6 +494,12 @@ __device__ __forceinline__ KerrSlope<R> kerr_slope(const KerrRays<R>& k, R r, R 
     return o;
 }
 
+// Whether ray j's state is five finite numbers.
+template <typename R> __device__ __forceinline__ bool finite_state(const KerrRays<R>& p, int j) {
+    const float sum = part(p.r, j) + part(p.th, j) + part(p.ph, j) + part(p.pr, j) + part(p.pt, j);
+    return fabsf(sum) < INFINITY;
+}
+
 // One step of every ray of the lane (march.metal:140-173), after `step`
 // others. Rays that ended stay where they are: their step length is zero.
 template <typename R, typename View>
@@ -597,10 +603,15 @@ __device__ __forceinline__ void kerr_step(KerrRays<R>& p, const View& u, uint32_
             if (!alive(sh, j) || (r > p.capture && r < u.escape)) continue;
             // A last step beside the horizon can leave a state that is no
             // number and would stay so to the step cap: it ends as one that
-            // got there, over its drift budget and so re-integrated in FP64.
+            // got there, with a drift over any budget and a radius inside any
+            // limit, so that it is re-integrated in FP64 (needs_fp64).
             const bool in = r <= p.capture;
             sh.end[j] = end_word(step + 1u, in ? RayCaptured : r >= u.escape ? RayEscaped : RayExhausted);
             sh.longest[j] = 0.0f;
+            if (!in && !finite_state(p, j)) {
+                p.gauge[j] = INFINITY;
+                sh.min_r[j] = 0.0f;
+            }
             if (in) p.gauge[j] = kerr_drift(kerr_lane(p, j));  // now: held inside the horizon, it need not stay finite
             // A step of length zero adds the error words: without them it moves nothing.
             R* words[5] = {&p.er, &p.eth, &p.eph, &p.epr, &p.ept};
@@ -636,8 +647,12 @@ __device__ __forceinline__ PixelResult kerr_finish(const KerrRays<R>& p, int j, 
     l.samples = j == 0 ? p.sh.samples : 0u;
     l.outcome = end_outcome(p.sh.end[j]);
     l.min_r = p.sh.min_r[j];
+    // A state that is no number gives no direction to look up a star in:
+    // written as it is (where the FP64 list is full), its ray finds none.
+    if (!finite_state(p, j)) l.outcome = RayCaptured;
     PixelResult r = kerr_pixel(l, u, blackbody);
-    if (l.outcome == RayCaptured) r.drift = p.gauge[j];
+    r.outcome = end_outcome(p.sh.end[j]);
+    if (r.outcome == RayCaptured) r.drift = p.gauge[j];
     return r;
 }
 

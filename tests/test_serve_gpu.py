@@ -479,3 +479,20 @@ def test_a_request_in_two_waves_is_the_same(world, width, height, cap, spin):
         assert waves == (2 if in_flight == 0 else 1)
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("wave_rays", [64, 0])  # the FP64 list of a 64-ray wave holds 8 rays: most are written as they are
+def test_rays_that_blow_up_leave_finite_pixels(world, wave_rays):
+    """Seven rays of this near-extremal image end beside the horizon in a
+    state that is no number. The star seed has a star in the cell that a
+    direction of no numbers falls into."""
+    import gargantua_b200 as g
+
+    spec = g.RequestSpec(640, 360, 4096, 0.998, azimuth=1.6648687, elevation=0.2479261, distance=33.6584625, fov_y=0.457963,
+                         star_seed=5)
+    server = g.Server(world["ctx"], world["vol"], g.types.SERVE_BATCHED, wave_rays=wave_rays,
+                      fp64_policy=g.types.FP64_ALL_FLAGGED)
+    pixels, _, res = server.wait(server.submit(spec))
+    server.close()
+    assert res.counters.rays == 640 * 360
+    assert np.isfinite(pixels.astype(np.float32)).all()
