@@ -24,11 +24,15 @@
 // and two to a lane they ran 1.35 times slower.
 //
 // Everything here is a template over R: F2 (two neighbouring pixels per
-// lane) or float (one ray per lane). The state advances operation by
-// operation as k_step's compiled code rounds it (lanes.cuh): every
-// multiply-add is written out as the fused or the separate operation it is
-// there, so the two give the same bits, and a ray's values do not depend on
-// the ray it shares a lane with.
+// lane) or float (one ray per lane). Radius, polar angle, their momenta and
+// the gauges advance operation by operation as k_step's compiled code rounds
+// them (lanes.cuh): every multiply-add is written out as the fused or the
+// separate operation it is there, so steps, outcomes and drifts are the image
+// march's bit for bit (tested), and a ray's values do not depend on the ray
+// it shares a lane with. The azimuth, which enters none of these, is not: the
+// compiler contracts its rate differently from kernel to kernel, and a
+// sample's place and path come from a series of their own (kerr_step);
+// colours differ in the last bits.
 #pragma once
 
 #include "lanes.cuh"
@@ -113,11 +117,14 @@ __device__ __forceinline__ float smallest(F2 a) {
     return fminf(p.x, p.y);
 }
 
-// fast_sincos of every ray's angle. k = rint(x 2/pi) comes from adding
-// 1.5 2^23, whose sum holds k in its low bits: no conversion instructions.
-template <typename R> __device__ __forceinline__ void sincos_of(R x, R* s_out, R* c_out) {
+// fast_sincos of every ray's angle, bit for bit up to |x| = 2^22 pi/2 (only a
+// state that blew up is beyond). k = rint(x 2/pi) comes from adding 1.5 2^23
+// to the rounded product, whose sum holds k in its low bits: no conversion
+// instructions. (Fused, near ties k is the other neighbour: of 635,000 rays
+// one ended with another drift.)
+template <typename R> __device__ __forceinline__ void sincos_of(R x, float minus_zero, R* s_out, R* c_out) {
     constexpr int N = Rays<R>::N;
-    const R kk = mad(x, all<R>(0.636619772367581f), all<R>(12582912.0f));
+    const R kk = add(product(x, all<R>(0.636619772367581f), minus_zero), all<R>(12582912.0f));
     const R k = add(kk, all<R>(-12582912.0f));
     R r = mad(k, all<R>(-1.57079601287841796875f), x);
     r = mad(k, all<R>(-3.13916478650481e-07f), r);
@@ -561,7 +568,7 @@ __device__ __forceinline__ void kerr_step(KerrRays<R>& p, const View& u, uint32_
     settle(p.ph, p.eph, bph, w, u);
     settle(p.pr, p.epr, bpr, w, u);
     settle(p.pt, p.ept, bpt, w, u);
-    sincos_of(p.th, &p.st, &p.ct);
+    sincos_of(p.th, u.minus_zero, &p.st, &p.ct);
     // The azimuth enters only a sample's position: its sine and cosine, and
     // the path since the previous state (the chord between the two in
     // cylinder coordinates, in which nothing cancels), are taken only near
@@ -569,7 +576,7 @@ __device__ __forceinline__ void kerr_step(KerrRays<R>& p, const View& u, uint32_
     const R z = mul(p.r, p.ct);
     if (smallest(magnitude(z)) < DISK_SLAB_HALF_HEIGHT && u.gas) {
         R sp, cp;
-        sincos_of(p.ph, &sp, &cp);
+        sincos_of(p.ph, u.minus_zero, &sp, &cp);
         const R rho = mul(asqrt(mad(p.r, p.r, all<R>(p.a2))), p.st);
         const R axial0 = asqrt(mad(r0, r0, all<R>(p.a2))), rho0 = mul(axial0, st0);
         const R out = mad(neg(axial0), st0, rho), up = mad(neg(r0), ct0, z);

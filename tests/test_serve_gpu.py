@@ -496,3 +496,62 @@ def test_rays_that_blow_up_leave_finite_pixels(world, wave_rays):
     server.close()
     assert res.counters.rays == 640 * 360
     assert np.isfinite(pixels.astype(np.float32)).all()
+
+
+def served_uniforms(spec):
+    """A request's uniforms in the server's own float32 operations: the C library's cosf, sinf and tanf."""
+    import ctypes as C
+
+    import gargantua_b200 as g
+
+    libm = C.CDLL("libm.so.6")
+    f = np.float32
+
+    def call(name, x):
+        fn = getattr(libm, name)
+        fn.restype, fn.argtypes = C.c_float, [C.c_float]
+        return f(fn(float(f(x))))
+
+    cam = g.OrbitCamera(spec.azimuth, spec.elevation, spec.distance, spec.fov_y)
+    c, d = call("cosf", spec.elevation), f(spec.distance)
+    p = [d * (c * call("cosf", spec.azimuth)), d * (c * call("sinf", spec.azimuth)), d * call("sinf", spec.elevation)]
+    inv = f(1) / np.sqrt(p[0] * p[0] + p[1] * p[1] + p[2] * p[2])
+    fx, fy, fz = (-v * inv for v in p)
+    rn = f(1) / np.sqrt(fy * fy + fx * fx)
+    rx, ry = fy * rn, -fx * rn
+    up = [ry * fz - f(0) * fy, f(0) * fx - rx * fz, rx * fy - ry * fx]
+    st = g.Settings.interactive() if spec.step_cap <= 256 else g.Settings.still()
+    st.step_cap = spec.step_cap
+    st.escape_radius = max(st.escape_radius, float(d + f(10)))
+    u = g.uniforms(cam, spec.width, spec.height, st, 1e9, True, spec.star_seed, spin=spec.spin)  # no FP64 pass
+    u.cameraPosition = g.types.Float3(*p, 0.0)
+    u.cameraRight = g.types.Float3(rx, ry, 0.0, 0.0)
+    u.cameraUp = g.types.Float3(*up, 0.0)
+    u.cameraForward = g.types.Float3(fx, fy, fz, 0.0)
+    t = call("tanf", f(spec.fov_y) * f(0.5))
+    u.tanHalfFov = g.types.Float2(t * f(spec.width) / f(spec.height), t)
+    return u
+
+
+@pytest.mark.parametrize("spin", [0.02, 0.5, 0.9, 0.998])
+@pytest.mark.parametrize("width,height", [(1101, 577), (333, 217)])  # two rays to a lane, and one
+def test_served_kerr_steps_are_the_image_march_s(world, width, height, spin):
+    """A served Kerr ray advances (pairs.cuh) as the compensated image march
+    advances it (lanes.cuh): the same step count, outcome and drift, bit for
+    bit. Left out are the rays that the server re-integrates in FP64 and
+    those whose state is no number, which it ends at once."""
+    import gargantua_b200 as g
+
+    spec = g.RequestSpec(width, height, 4096, spin, azimuth=0.8, elevation=0.15, distance=46.0)
+    server = g.Server(world["ctx"], world["vol"], g.types.SERVE_BATCHED)
+    _, served, res = server.wait(server.submit(spec, debug=True))
+    server.close()
+    t = g.Targets(world["ctx"], width, height)
+    g.march(world["ctx"], world["vol"], served_uniforms(spec), t, g.types.PRECISION_COMPENSATED)
+    _, image, _ = t.read()
+    t.close()
+    drift, outcome = image[:, 0].astype(np.float32), image[:, 2].astype(np.float32)
+    over = (drift > 0.99e-5) & (outcome != 0)  # over the still's budget, not captured: FP64 if it passed close
+    assert over.mean() < 0.2 and res.fp64_rays <= over.sum()
+    differ = np.any(served.view(np.uint16)[~over, :3] != image.view(np.uint16)[~over, :3], axis=1)
+    assert not differ.any(), int(differ.sum())
