@@ -242,6 +242,21 @@ template <typename R> __device__ __forceinline__ V3<R> s_direction(const SLane<R
     return len2 > R(0) ? local * rsqrtT(len2) : radial;
 }
 
+// Everything of a ray that its first step finds besides its state l.s and what is constant.
+template <typename R> __device__ __forceinline__ void s_begin(SLane<R>& l) {
+    l.c = SState<R>{R(0), R(0), R(0), R(0), R(0)};
+    l.pre_drift = 0.0f;
+    l.color = make_float3(0.0f, 0.0f, 0.0f);
+    l.transmittance = 1.0f;
+    l.travelled = l.weighted_depth = l.depth_weight = 0.0f;
+    R sn, cs;
+    l.previous = s_position(l, &sn, &cs);
+    l.steps = l.samples = 0;
+    l.outcome = RayExhausted;
+    l.min_r = (float)l.s.r;
+    l.left_sphere = false;
+}
+
 // prepareRay (Geodesic.h:130-163) into a lane. Returns true when the ray is
 // sky-only; then *sky holds its asymptotic direction.
 template <typename R>
@@ -257,20 +272,10 @@ __device__ __forceinline__ bool s_init(SLane<R>& l, V3<R> origin, V3<R> directio
         return true;
     }
     l.s = SState<R>{p.ray.s.r, p.ray.s.phi, p.ray.s.vDot, p.ray.s.rDot, p.ray.s.phiDot};
-    l.c = SState<R>{R(0), R(0), R(0), R(0), R(0)};
     double r0 = (double)l.s.r;
     l.e0 = (1.0 - 2.0 / r0) * (double)l.s.vd - (double)l.s.rd;
     l.l0 = r0 * r0 * (double)l.s.pd;
-    l.pre_drift = 0.0f;
-    l.color = make_float3(0.0f, 0.0f, 0.0f);
-    l.transmittance = 1.0f;
-    l.travelled = l.weighted_depth = l.depth_weight = 0.0f;
-    R sn, cs;
-    l.previous = s_position(l, &sn, &cs);
-    l.steps = l.samples = 0;
-    l.outcome = RayExhausted;
-    l.min_r = (float)l.s.r;
-    l.left_sphere = false;
+    s_begin(l);
     return false;
 }
 
@@ -437,11 +442,14 @@ __device__ __forceinline__ float s_inner(const MarchUniforms& u) {
 
 // A ray from its launch to its end, as s_step takes it. A landing on the
 // sphere needs the state its step set out from; keeping that copies the ten
-// words of the state each step. So the steps inside s_inner, which cannot
+// words of the state each step. So the steps inside s_inner, which should not
 // reach the sphere, have a loop of their own without it (a 1920x1080 still's
-// kernel: 1070 -> 1020 us; the live image's 960x540: 331 -> 313). A state
-// that blew up at the hole may cross both radii at once; it has left then,
-// without landing. Both loops take at most the step budget.
+// kernel: 1070 -> 1020 us; the live image's 960x540: 331 -> 313). Steps too
+// long for the field, or a state that blew up at the hole, may cross both
+// radii at once: such a ray ends with min_r = kUnlanded, and its caller
+// marches it again with s_step or in FP64. Both loops take at most the step
+// budget.
+constexpr float kUnlanded = -INFINITY;
 template <bool Comp>
 __device__ __forceinline__ void s_march(SLane<float>& l, const MarchUniforms& u, cudaTextureObject_t em,
                                         cudaTextureObject_t vel, bool gather) {
@@ -461,6 +469,7 @@ __device__ __forceinline__ void s_march(SLane<float>& l, const MarchUniforms& u,
             if (left || l.s.r >= g.escapeRadius) {
                 l.outcome = RayEscaped;
                 l.left_sphere = left;
+                if (left) l.min_r = kUnlanded;
                 return;
             }
         }
@@ -959,11 +968,15 @@ __device__ inline PixelResult shade_pixel_lane(const MarchParams& p, uint32_t px
     float3 sky;
     if (s_init(l, origin, dir, u, p.tables, &sky)) return sky_only_result(sky, u, p.blackbody);
     if constexpr (sizeof(R) == 4 && !Project) {
+        // volatile: kept in memory, where it costs the steps no registers
+        volatile float launch[5] = {l.s.r, l.s.phi, l.s.vd, l.s.rd, l.s.pd};
         s_march<Comp>(l, u, p.emission, p.velocity, gather);
-    } else {
-        for (uint32_t k = 0; k <= STEP_CAP_STILL; ++k)
-            if (s_step<R, Comp, Project>(l, u, p.emission, p.velocity, gather)) break;
+        if (l.min_r != kUnlanded) return s_finish(l, u, p.tables, p.blackbody);
+        l.s = SState<float>{launch[0], launch[1], launch[2], launch[3], launch[4]};
+        s_begin(l);
     }
+    for (uint32_t k = 0; k <= STEP_CAP_STILL; ++k)
+        if (s_step<R, Comp, Project>(l, u, p.emission, p.velocity, gather)) break;
     return s_finish(l, u, p.tables, p.blackbody);
 }
 

@@ -296,6 +296,7 @@ __device__ void serve_schwarzschild_chunks(const WaveArgs& a, uint32_t lane) {
                 } else {
                     s_march<true>(L, u, em, vel, em != 0);
                     r = s_finish(L, u, t, a.blackbody);
+                    if (r.min_r == kUnlanded) r.drift = INFINITY;  // to FP64
                     complete(a, ch.request, pixel, r);
                 }
             }

@@ -61,3 +61,30 @@ def test_block_shape_refusals_and_autotune(scene):
     tuned = autotune.tune_march_block(ctx, vol, u, blocks=((8, 8), (32, 4)), repeats=1)
     assert tuned["block"] in ([8, 8], [32, 4]) and tuned["ms"] > 0.0 and len(tuned["trials"]) == 2
     ctx.set_march_block(8, 8)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("factor,longest", [(1.5, 5.0), (0.02, 0.5)])  # steps too long for the field; the defaults
+def test_image_rays_land_as_probes_do(scene, precision, factor, longest):
+    """The image march takes the steps that should not reach the sphere in a
+    loop without the landing, the probes every step with it. Steps so long
+    that a ray at r = 5 lands beyond r = 30 give the same counts, outcomes
+    and drifts in both."""
+    import gargantua_b200 as g
+
+    ctx, _ = scene
+    st = g.Settings(600, step_factor=factor, step_max=longest, empty_step_factor=0.06, empty_step_max=longest)
+    t = g.Targets(ctx, 1, 1)
+    got, want = [], []
+    for b in np.linspace(5.01, 5.11, 41):
+        origin = np.array([np.sqrt(40.0 ** 2 - b * b), b, 0.0], np.float32)
+        u = g.uniforms(g.OrbitCamera(), 1, 1, st, 1e9, False, 1, stars=False)
+        u.cameraPosition = g.types.Float3(*origin, 0.0)
+        u.cameraForward = g.types.Float3(-1.0, 0.0, 0.0, 0.0)
+        ctx.enable_tables(u, 40.0)
+        g.march(ctx, None, u, t, precision)
+        got.append(t.read()[1][0, :3].astype(np.float32))
+        r = ctx.probe([g.Launch(origin.astype(np.float64), np.array([-1.0, 0.0, 0.0]))], u, precision)
+        want.append([np.float16(r["drift"][0]), r["steps"][0], r["outcome"][0]])
+    t.close()
+    assert np.array_equal(np.array(got), np.array(want, np.float32), equal_nan=True)
