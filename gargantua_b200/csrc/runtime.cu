@@ -42,6 +42,7 @@ int device_alloc(gg_context* ctx, uint64_t bytes, void** out, const char* what) 
                     (unsigned long long)bytes, (unsigned long long)(ctx->budget - ctx->used),
                     (unsigned long long)ctx->budget);
     }
+    make_room(ctx, bytes);
     GG_CUDA(cudaMalloc(out, bytes), what);
     ctx->used += bytes;
     return GG_OK;
@@ -51,6 +52,29 @@ void device_free(gg_context* ctx, void* ptr, uint64_t bytes) {
     if (!ptr) return;
     cudaFree(ptr);
     ctx->used -= bytes < ctx->used ? bytes : ctx->used;
+}
+
+static void drop_records(gg_context* ctx) {
+    cudaFree(ctx->record_buffer);
+    ctx->record_buffer = nullptr;
+    ctx->record_capacity = 0;
+}
+
+void make_room(gg_context* ctx, uint64_t bytes) {
+    if (ctx->record_buffer && ctx->used + bytes + ctx->record_capacity > ctx->budget) drop_records(ctx);
+}
+
+void* record_scratch(gg_context* ctx, uint64_t bytes) {
+    if (ctx->record_capacity >= bytes) return ctx->record_buffer;
+    drop_records(ctx);
+    if (ctx->used + bytes > ctx->budget) return nullptr;
+    if (cudaMalloc(&ctx->record_buffer, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->record_buffer = nullptr;
+        return nullptr;
+    }
+    ctx->record_capacity = bytes;
+    return ctx->record_buffer;
 }
 
 int ensure_capacity(gg_context* ctx, void** ptr, uint64_t* capacity, uint64_t bytes, const char* what) {
@@ -250,6 +274,7 @@ GG_API void gg_context_destroy(gg_context* ctx) {
     cudaFree(ctx->counters);
     cudaFree(ctx->stats);
     cudaFree(ctx->probe_buffer);
+    cudaFree(ctx->record_buffer);
     cudaFree(ctx->flagged);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;

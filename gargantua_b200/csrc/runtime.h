@@ -89,6 +89,9 @@ struct gg_context {
     uint32_t march_block_h = MARCH_THREADGROUP_HEIGHT;
     void* probe_buffer = nullptr;
     uint64_t probe_capacity = 0;  // bytes
+    // Idle between readbacks; not in `used`, but never beyond the budget with it (make_room).
+    void* record_buffer = nullptr;
+    uint64_t record_capacity = 0;  // bytes
     uint32_t* flagged = nullptr;  // FP64 re-integration list
     uint64_t flagged_capacity = 0;  // entries
 };
@@ -101,6 +104,12 @@ namespace gg {
 int device_alloc(gg_context* ctx, uint64_t bytes, void** out, const char* what);
 void device_free(gg_context* ctx, void* ptr, uint64_t bytes);
 int ensure_capacity(gg_context* ctx, void** ptr, uint64_t* capacity, uint64_t bytes, const char* what);
+// Device scratch for a readback's records, kept for the next one while the
+// budget has room for it; null where it has not (no error is set).
+void* record_scratch(gg_context* ctx, uint64_t bytes);
+// Called before `bytes` join `used`: gives the record scratch back if the
+// budget does not hold both.
+void make_room(gg_context* ctx, uint64_t bytes);
 
 // Host-side table construction (FP64, then rounded), the work
 // ParticleSystem.init does on the host (ParticleSystem.swift:23-47).

@@ -1159,6 +1159,7 @@ GG_API int gg_server_create(gg_context* ctx, const gg_volume* vol, const gg_serv
         if (s->cfg.schedule == GG_SCHEDULE_CHUNKS) GG_CHECK(gg::capture_wave_graph(s.get(), w, true));
     }
     GG_CUDA(cudaStreamSynchronize(s->build), "server set-up");
+    make_room(ctx, s->cfg.memory_bytes);
     ctx->used += s->cfg.memory_bytes;  // reserved for admitted requests
     s->worker = std::thread(gg::worker_loop, s.get());
     *out = s.release();

@@ -755,6 +755,7 @@ GG_API int gg_volume_create(gg_context* ctx, uint32_t size, gg_volume** out) {
     if (ctx->used + sums_bytes + tex_bytes > ctx->budget)
         return gg::fail(GG_ERR_OVER_BUDGET, "A %u^3 volume needs %llu bytes but the budget has %llu bytes left.", size,
                         (unsigned long long)(sums_bytes + tex_bytes), (unsigned long long)(ctx->budget - ctx->used));
+    gg::make_room(ctx, sums_bytes + tex_bytes);
     gg_volume* vol = new gg_volume();
     vol->ctx = ctx;
     vol->size = size;

@@ -142,7 +142,9 @@ GG_API int gg_particles_step(gg_particles* ps, uint32_t dispatches);
 
 /* Copy the state out as ShaderTypes Particle records (32 bytes each) into a
  * host array of `count` entries (count must equal the system's count).
- * Replaces Validate.readback (Validate.swift:88-100). */
+ * Replaces Validate.readback (Validate.swift:88-100). Takes nothing from the
+ * context's budget: the records are packed on the device in up to 16 MB that
+ * the budget has left, which go as soon as something else needs them. */
 GG_API int gg_particles_read(gg_particles* ps, Particle* out, uint32_t count);
 
 /* Replace the device state with `count` host Particle records. */

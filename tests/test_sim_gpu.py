@@ -195,3 +195,29 @@ def test_records_are_read_without_budget_for_packing():
     assert ctx.memory()[1] <= ctx.memory()[0]
     ps.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("spare,size", [(1 << 20, 24), (5 << 20, 48)])  # less room than a read's scratch, and more
+def test_a_read_leaves_the_budget_as_it_found_it(spare, size):
+    """Particles read back take nothing from the context's budget: a volume
+    that fitted before a read fits after it, the probes' scratch is still
+    there, and a read that succeeds leaves no error sentence."""
+    import gargantua_b200 as g
+
+    with g.Context() as probe:
+        base = probe.memory()[1]
+    count = 100_000
+    with g.Context(0, budget_bytes=base + count * 32 + 4096 + spare) as ctx:
+        ps = g.Particles(ctx, count, seed=3)
+        ps.seed_particles()
+        u = g.uniforms(g.OrbitCamera(), 1, 1, g.Settings.interactive(), 1e-4, False, 0, spin=0.5)
+        launches = g.camera_grid(g.OrbitCamera(), 4, 4, 1.0)
+        ctx.probe(launches, u)
+        with pytest.raises(g.GargantuaError):
+            g.Targets(ctx, 4096, 4096)  # a sentence of its own
+        used, sentence = ctx.memory()[1], g.lib().gg_last_error()
+        first = ps.read()
+        assert ctx.memory()[1] == used and g.lib().gg_last_error() == sentence
+        g.Volume(ctx, size).close()  # 0.6 of 1 MB, 4.4 of 5 MB
+        assert np.array_equal(ps.read().view(np.uint32), first.view(np.uint32))
+        ctx.probe(launches, u)
