@@ -576,13 +576,14 @@ class Bake:
     def bake_rows(self, u: T.MarchUniforms, row_begin: int, row_end: int):
         check(lib().gg_bake_rows(self.handle, C.byref(u), row_begin, row_end))
 
-    def bake_full(self, u: T.MarchUniforms, frames: int = 4):
-        """encodeFullBake (BakePass.swift:55-84): every row. The reference
-        encodes BAKE_FRAMES chunks of rows, one a frame; issued together, as
-        here, they are one launch whatever `frames` is: at the end of each of
-        four the device waited for its longest rays (960x540: 774 us, one
-        launch 516 us)."""
-        self.bake_rows(u, 0, self.height)
+    def bake_full(self, u: T.MarchUniforms, frames: int = 1):
+        """encodeFullBake (BakePass.swift:55-84): every row, in launches of
+        height // frames rows. The reference encodes BAKE_FRAMES = 4 chunks,
+        one a frame; issued together they end four times on their longest
+        rays (960x540: 774 us, one launch 516 us)."""
+        rows = max(self.height // frames, 1)
+        for r in range(0, self.height, rows):
+            self.bake_rows(u, r, min(r + rows, self.height))
 
     def overflow(self, reset: bool = False) -> int:
         c = C.c_uint32()

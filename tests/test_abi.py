@@ -209,3 +209,22 @@ def test_swift_module_files_bind_the_header():
     declared = set(re.findall(r"GG_API\s+(?:const\s+)?\w+\s*\**\s*(gg_\w+)\(", header))
     called = set(re.findall(r"\b(gg_\w+)\(", open(os.path.join(swift, "Sources", "gg-still", "main.swift")).read()))
     assert called and called <= declared, called - declared
+
+
+@pytest.mark.parametrize("height,frames,rows", [
+    (10, None, [(0, 10)]), (10, 1, [(0, 10)]), (8, 4, [(0, 2), (2, 4), (4, 6), (6, 8)]),
+    (10, 4, [(0, 2), (2, 4), (4, 6), (6, 8), (8, 10)]), (2, 4, [(0, 1), (1, 2)])])
+def test_a_full_bake_issues_the_launches_it_is_asked_for(height, frames, rows):
+    """Bake.bake_full: `frames` chunks of rows (BakePass.swift:55-84), one launch unless asked."""
+    import gargantua_b200 as g
+
+    class Recorder:
+        def __init__(self):
+            self.height, self.calls = height, []
+
+        def bake_rows(self, u, begin, end):
+            self.calls.append((begin, end))
+
+    r = Recorder()
+    g.Bake.bake_full(r, None) if frames is None else g.Bake.bake_full(r, None, frames)
+    assert r.calls == rows
