@@ -39,6 +39,7 @@
 
 #include "pairs.cuh"
 #include "runtime.h"
+#include "waves.h"
 
 namespace gg {
 
@@ -419,7 +420,6 @@ __global__ void __launch_bounds__(kServeThreads, kServeBlocksPerSM) serve_kerr_s
 
 // FP64 re-integration of the wave's flagged rays.
 constexpr uint32_t kReintegratePerWarp = 8;
-constexpr uint32_t kSpareBlocks = 40;  // the FP64 pass of a 1920x1080 still: 1280 rays, 8 to a warp
 
 __global__ void __launch_bounds__(128) serve_reintegrate_kernel(WaveArgs a) {
     const uint32_t n = min(a.header->flagged_count, a.flagged_capacity);
@@ -571,7 +571,7 @@ struct gg_server {
     uint64_t next_ticket = 1;
     uint64_t memory_used = 0;
     bool kerr_single = false;  // the last wave formed has one Kerr ray to a lane
-    bool parted = false;  // the last wave formed was the first part of two (form_wave)
+    uint64_t parted_rest = 0;  // rays left for the second part of a request just parted in two (form_wave)
     bool stop = false;
     int fatal = GG_OK;
     std::string fatal_sentence;
@@ -762,7 +762,9 @@ static bool form_wave(gg_server* s, WaveSlot& w) {
         if (r->u.spin > 0.0f) kerr_rays += r->rays - r->next_ray;
     kerr_rays = std::min<uint64_t>(kerr_rays, s->cfg.wave_rays);
     const bool busy = std::any_of(s->slots.begin(), s->slots.end(), [](const WaveSlot& o) { return o.busy; });
-    const bool second = s->parted && busy;
+    uint64_t left = 0;
+    for (auto& r : cands) left += r->rays - r->next_ray;
+    const bool second = busy && s->parted_rest != 0 && left == s->parted_rest;  // the rest and nothing else
     s->kerr_single = s->cfg.schedule == GG_SCHEDULE_CHUNKS && !(second && !s->kerr_single) &&
                      kerr_rays < 3ull * 64u * (uint64_t)s->grid_k * (kServeThreads / 32);
     w.kerr_single = s->kerr_single;
@@ -770,22 +772,20 @@ static bool form_wave(gg_server* s, WaveSlot& w) {
     // Kerr rays that would make one last wave, with nothing else under way,
     // make two: the rays flagged for FP64 pass close to the hole, so they are
     // among the first two fifths (ray_pixel), and that part's FP64 pass, a
-    // millisecond of latency, runs beside the rest, which leaves it the places
-    // of kSpareBlocks blocks. Lone stills: 640x360 1380 -> 1190 us (256 steps)
+    // millisecond of latency, runs beside the rest, which leaves it some places
+    // (spare_blocks). Lone stills: 640x360 1380 -> 1190 us (256 steps)
     // and 2210 -> 2120 (4096), 960x540 2260 -> 2080 and 3100 -> 2630,
     // 1280x720 7080 -> 5970 (4096), 1920x1080 7080 -> 6230. The line is at one
     // round of rays: below it the wave's end is that of its longest rays, and
     // two waves end 1 to 2 % later.
     uint64_t budget = s->cfg.wave_rays;
+    s->parted_rest = 0;
     if (second) {
-        hdr->spare_blocks = kSpareBlocks;
-        s->parted = false;
-    } else {
-        uint64_t left = 0;
-        for (auto& r : cands) left += r->rays - r->next_ray;
-        s->parted = !busy && s->slots.size() > 1 && s->cfg.schedule == GG_SCHEDULE_CHUNKS && left <= budget &&
-                    kerr_rays >= (uint64_t)s->grid_k1 * kServeThreads;
-        if (s->parted) budget = left * 2u / 5u & ~63ull;
+        hdr->spare_blocks = spare_blocks((uint32_t)(w.kerr_single ? s->grid_k1 : s->grid_k));
+    } else if (!busy && s->slots.size() > 1 && s->cfg.schedule == GG_SCHEDULE_CHUNKS && left <= budget &&
+               kerr_rays >= (uint64_t)s->grid_k1 * kServeThreads) {
+        budget = left * 2u / 5u & ~63ull;
+        s->parted_rest = left - budget;
     }
     w.members.clear();
     std::vector<uint32_t> local(cands.size(), UINT32_MAX);

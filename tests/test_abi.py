@@ -228,3 +228,18 @@ def test_a_full_bake_issues_the_launches_it_is_asked_for(height, frames, rows):
     r = Recorder()
     g.Bake.bake_full(r, None) if frames is None else g.Bake.bake_full(r, None, frames)
     assert r.calls == rows
+
+
+def test_the_fp64_pass_leaves_a_wave_its_places(tmp_path):
+    """The blocks that a request's second wave gives up (csrc/waves.h) are
+    never more than an eighth of its grid, whatever the device's size."""
+    import subprocess
+
+    src = tmp_path / "t.cpp"
+    src.write_text('#include "waves.h"\nint main() { for (unsigned g = 0; g < 5000; ++g) '
+                   "if (gg::spare_blocks(g) * 8 > g || gg::spare_blocks(g) > 40) return 1; "
+                   "return gg::spare_blocks(592) == 40 ? 0 : 2; }\n")
+    r = subprocess.run(["/usr/bin/g++", "-std=c++17", str(src), "-I", os.path.join(ROOT, "gargantua_b200", "csrc"),
+                        "-o", str(tmp_path / "t")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    assert subprocess.run([str(tmp_path / "t")]).returncode == 0
