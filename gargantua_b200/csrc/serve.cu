@@ -536,8 +536,11 @@ struct WaveSlot {
     cudaEvent_t fork = nullptr, join = nullptr;
     cudaEvent_t fp64_done = nullptr;
     cudaEvent_t start = nullptr, stop = nullptr;
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};  // with Kerr rays two to a lane, and one
-    bool kerr_single = false;                       // the wave being formed takes graph[1]
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    cudaGraphNode_t kerr_node = nullptr;
+    bool exec_single = false;  // exec's Kerr kernel has one ray to a lane (chunk schedule)
+    bool kerr_single = false;  // the wave being formed wants it to
     char* device = nullptr;  // header, requests, chunks0, chunks1, flagged
     char* host = nullptr;    // pinned staging for the descriptors
     bool busy = false;
@@ -594,11 +597,9 @@ static uint64_t slot_offset_chunks1(const gg_server* s) { return slot_offset_chu
 static uint64_t slot_offset_flagged(const gg_server* s) { return slot_offset_chunks1(s) + (uint64_t)s->max_chunks * sizeof(ServeChunk); }
 
 // The wave graph: fork, the Schwarzschild and Kerr persistent kernels side
-// by side, join; a slot has one for each Kerr kernel of its schedule. The
-// FP64 pass is launched outside the graph on its own stream so it overlaps
-// the next wave.
-static int capture_wave_graph(gg_server* s, WaveSlot& w, bool single) {
-    cudaGraph_t g = nullptr;
+// by side, join. The FP64 pass is launched outside the graph on its own
+// stream so it overlaps the next wave.
+static int capture_wave_graph(gg_server* s, WaveSlot& w) {
     GG_CUDA(cudaStreamBeginCapture(w.stream, cudaStreamCaptureModeThreadLocal), "wave capture");
     GG_CUDA(cudaEventRecord(w.fork, w.stream), "wave capture");
     GG_CUDA(cudaStreamWaitEvent(w.side, w.fork, 0), "wave capture");
@@ -607,16 +608,32 @@ static int capture_wave_graph(gg_server* s, WaveSlot& w, bool single) {
         serve_kerr_kernel<<<s->grid_k, kServeThreads, 0, w.stream>>>(w.args);
     } else {
         serve_schwarzschild_chunks_kernel<<<s->grid_s, kServeThreads, 0, w.side>>>(w.args);
-        if (single) serve_kerr_single_chunks_kernel<<<s->grid_k1, kServeThreads, 0, w.stream>>>(w.args);
-        else serve_kerr_chunks_kernel<<<s->grid_k, kServeThreads, 0, w.stream>>>(w.args);
+        serve_kerr_chunks_kernel<<<s->grid_k, kServeThreads, 0, w.stream>>>(w.args);
     }
+    cudaStreamCaptureStatus status;
+    const cudaGraphNode_t* last = nullptr;
+    size_t lasts = 0;
+    GG_CUDA(cudaStreamGetCaptureInfo_v2(w.stream, &status, nullptr, nullptr, &last, &lasts), "wave capture");
+    if (lasts == 1) w.kerr_node = last[0];
     GG_CUDA(cudaEventRecord(w.join, w.side), "wave capture");
     GG_CUDA(cudaStreamWaitEvent(w.stream, w.join, 0), "wave capture");
-    cudaError_t e = cudaStreamEndCapture(w.stream, &g);
-    GG_CUDA(e, "wave capture");
-    e = cudaGraphInstantiate(&w.graph[single ? 1 : 0], g, 0);
-    cudaGraphDestroy(g);
-    GG_CUDA(e, "wave graph instantiate");
+    GG_CUDA(cudaStreamEndCapture(w.stream, &w.graph), "wave capture");
+    GG_CUDA(cudaGraphInstantiate(&w.exec, w.graph, 0), "wave graph instantiate");
+    return w.kerr_node ? GG_OK : fail(GG_ERR_DEVICE, "wave capture: the Kerr kernel's node is not known.");
+}
+
+// The slot's graph with the Kerr kernel its wave wants. The slot is idle:
+// its last launch of the graph has completed.
+static int choose_kerr_kernel(gg_server* s, WaveSlot& w) {
+    if (w.kerr_single == w.exec_single) return GG_OK;
+    void* params[1] = {&w.args};
+    cudaKernelNodeParams k{};
+    k.func = w.kerr_single ? (void*)serve_kerr_single_chunks_kernel : (void*)serve_kerr_chunks_kernel;
+    k.gridDim = dim3(w.kerr_single ? s->grid_k1 : s->grid_k);
+    k.blockDim = dim3(kServeThreads);
+    k.kernelParams = params;
+    GG_CUDA(cudaGraphExecKernelNodeSetParams(w.exec, w.kerr_node, &k), "wave graph update");
+    w.exec_single = w.kerr_single;
     return GG_OK;
 }
 
@@ -836,6 +853,7 @@ static bool form_wave(gg_server* s, WaveSlot& w) {
 static int launch_wave(gg_server* s, WaveSlot& w) {
     gg::Range range("serve: launch wave");
     WaveHeader* hdr = reinterpret_cast<WaveHeader*>(w.host);
+    GG_CHECK(choose_kerr_kernel(s, w));
     GG_CUDA(cudaStreamWaitEvent(w.stream, s->built, 0), "wave ordering");
     GG_CUDA(cudaMemcpyAsync(w.device, w.host, sizeof(WaveHeader) + hdr->request_count * sizeof(ServeRequest),
                             cudaMemcpyHostToDevice, w.stream),
@@ -849,7 +867,7 @@ static int launch_wave(gg_server* s, WaveSlot& w) {
                                 hdr->chunk_count[1] * sizeof(ServeChunk), cudaMemcpyHostToDevice, w.stream),
                 "wave upload");
     GG_CUDA(cudaEventRecord(w.start, w.stream), "wave event");
-    GG_CUDA(cudaGraphLaunch(w.graph[w.kerr_single ? 1 : 0], w.stream), "wave launch");
+    GG_CUDA(cudaGraphLaunch(w.exec, w.stream), "wave launch");
     GG_CUDA(cudaEventRecord(w.stop, w.stream), "wave event");
     // FP64 pass after the wave, on its own stream: it overlaps the next wave.
     GG_CUDA(cudaStreamWaitEvent(w.fp64, w.stop, 0), "FP64 ordering");
@@ -1155,8 +1173,7 @@ GG_API int gg_server_create(gg_context* ctx, const gg_volume* vol, const gg_serv
         w.args.steps_per_round = s->cfg.steps_per_round;
         w.args.refill_idle = s->cfg.refill_idle;
         w.args.minus_zero = -0.0f;
-        GG_CHECK(gg::capture_wave_graph(s.get(), w, false));
-        if (s->cfg.schedule == GG_SCHEDULE_CHUNKS) GG_CHECK(gg::capture_wave_graph(s.get(), w, true));
+        GG_CHECK(gg::capture_wave_graph(s.get(), w));
     }
     GG_CUDA(cudaStreamSynchronize(s->build), "server set-up");
     make_room(ctx, s->cfg.memory_bytes);
@@ -1191,8 +1208,8 @@ void release_server_resources(gg_server* s) {
     for (auto& w : s->slots) {
         if (w.stream) cudaStreamSynchronize(w.stream);
         if (w.fp64) cudaStreamSynchronize(w.fp64);  // the FP64 pass reads the slot's flagged list
-        for (cudaGraphExec_t g : w.graph)
-            if (g) cudaGraphExecDestroy(g);
+        if (w.exec) cudaGraphExecDestroy(w.exec);
+        if (w.graph) cudaGraphDestroy(w.graph);
         if (w.device) gg::device_free(ctx, w.device, s->slot_bytes);
         if (w.host) cudaFreeHost(w.host);
         if (w.start) cudaEventDestroy(w.start);

@@ -555,3 +555,19 @@ def test_served_kerr_steps_are_the_image_march_s(world, width, height, spin):
     assert over.mean() < 0.2 and res.fp64_rays <= over.sum()
     differ = np.any(served.view(np.uint16)[~over, :3] != image.view(np.uint16)[~over, :3], axis=1)
     assert not differ.any(), int(differ.sum())
+
+
+def test_a_slot_changes_its_kerr_kernel_between_waves(world):
+    """One wave in flight: the slot's graph takes the kernel with one ray to a
+    lane, the one with two, and the first again."""
+    import gargantua_b200 as g
+
+    small = g.RequestSpec(160, 90, 4096, 0.9, azimuth=0.2, elevation=0.1, distance=40.0)
+    large = g.RequestSpec(1101, 577, 256, 0.9, azimuth=0.8, elevation=0.15, distance=46.0)
+    server = g.Server(world["ctx"], world["vol"], g.types.SERVE_BATCHED, max_waves_in_flight=1)
+    got = [run(server, [spec], debug=True)[0] for spec in (small, large, small, large)]
+    server.close()
+    for a, b in ((got[0], got[2]), (got[1], got[3])):
+        assert np.array_equal(a[0].view(np.uint16), b[0].view(np.uint16))
+        assert np.array_equal(a[1].view(np.uint16), b[1].view(np.uint16))
+        assert a[2].ray_steps == b[2].ray_steps and bytes(a[2].counters) == bytes(b[2].counters)
