@@ -571,3 +571,21 @@ def test_a_slot_changes_its_kerr_kernel_between_waves(world):
         assert np.array_equal(a[0].view(np.uint16), b[0].view(np.uint16))
         assert np.array_equal(a[1].view(np.uint16), b[1].view(np.uint16))
         assert a[2].ray_steps == b[2].ray_steps and bytes(a[2].counters) == bytes(b[2].counters)
+
+
+def test_schedules_give_the_same_bits_in_a_mix(world):
+    """Requests of both metrics and several spins in the same waves: the
+    chunk schedule, where a warp marches one request, and lane refill, where
+    its lanes march several, give equal pixels, debug targets and counters."""
+    import gargantua_b200 as g
+
+    out = []
+    for sch in (g.types.SCHEDULE_CHUNKS, g.types.SCHEDULE_LANE_REFILL):
+        server = g.Server(world["ctx"], world["vol"], g.types.SERVE_BATCHED, schedule=sch)
+        out.append(run(server, mix_specs() + [g.RequestSpec(1101, 577, 256, 0.9, elevation=0.2)], debug=True))
+        server.close()
+    for (pa, da, ra), (pb, db, rb) in zip(*out):
+        assert np.array_equal(pa.view(np.uint16), pb.view(np.uint16))
+        assert np.array_equal(da.view(np.uint16), db.view(np.uint16))
+        assert (ra.ray_steps, ra.samples, ra.fp64_rays) == (rb.ray_steps, rb.samples, rb.fp64_rays)
+        assert bytes(ra.counters) == bytes(rb.counters)
