@@ -288,8 +288,9 @@ def cpu_sample(slices, seconds: float, threads: int):
 
 def drift_vs_oracle(ctx, slices, per_request: int = 64, max_requests: int = 24) -> dict:
     """4096-step rays of the timed requests, 64 per request from a 64x36 grid
-    of its camera: drift of the compensated FP32 march (gg_probe, the served
-    arithmetic, FP64 re-integration off) beside the FP64 oracle's drift for
+    of its camera: drift of the compensated FP32 march (gg_probe, whose rays'
+    steps and drifts the served ones equal bit for bit, tested; FP64
+    re-integration off) beside the FP64 oracle's drift for
     the same rays (Schwarzschild: E and L; Kerr: Carter constant and null
     residual, each the maximum over the ray's steps as the reference
     defines it)."""

@@ -8,13 +8,15 @@
 // one issue slot and two cycles of the FMA pipe (measured: 2.06 cycles a
 // warp for fma, add and mul), so with two rays in a lane the arithmetic
 // takes half the issue slots. Min, max, selects, reciprocals and square
-// roots have no packed form and run once per ray. A ray step then issues 279
+// roots have no packed form and run once per ray. A ray step then issues 249
 // instructions, the azimuth's sine and cosine and the path taken only near
-// the slab. What bounds it now is latency and the mix of the pipes: 16 warps
-// per SM (126 registers) keep the FMA pipe 69 % and the issue slots 64 %
-// busy; 20 warps (96 registers, spilled) were slower, as was the RK4 loop
-// rolled. Measured on a 1920x1080 4096-step Kerr still: 6.55 -> 5.85 ms; on
-// the mixed served stream 79.5 -> 95 G ray-steps/s. (Hamilton's equations in
+// the slab. What bounds it now is the FMA pipe, on which a packed instruction
+// takes two cycles, and latency: 16 warps per SM (128 registers) keep the
+// pipe 71 % and the issue slots 62 % busy; 20 warps (96 registers, spilled)
+// were slower, as was the RK4 loop rolled. Measured on a 1920x1080 4096-step
+// Kerr still in one wave: 6.55 -> 5.54 ms, of which 5.85 before the rays went
+// through the image in tiles; on the mixed served stream 79.5 -> 95 G
+// ray-steps/s. (Hamilton's equations in
 // 32 operations instead of 40 and the RK4 sum in its final weights reached
 // 5.35 ms and 103 G, but round differently, and a ray's last bit decides
 // which cell of the starfield it meets.)

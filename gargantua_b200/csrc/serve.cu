@@ -1,21 +1,21 @@
 // Serving: continuous batching of still requests onto the device.
 //
-// Device side. A wave is one persistent launch over a queue of ray chunks
-// (chunk_rays consecutive pixels of one request) packed from every admitted
-// request, with one queue per metric: Schwarzschild rays and Kerr rays run
-// different integrators, so a warp works one queue at a time (half the
-// warps start on each, then take the other). Each warp steals chunks with
-// one atomic per chunk and runs its rays to their ends, two neighbouring
+// Device side. A wave is two queues of ray chunks (chunk_rays consecutive
+// rays of one request), packed from every admitted request, and a persistent
+// kernel for each, side by side: Schwarzschild rays and Kerr rays run
+// different integrators. Each warp steals chunks with one atomic per chunk
+// and runs its rays to their ends, two neighbouring
 // Kerr rays to a lane (pairs.cuh); under the lane-refill schedule a lane
 // whose ray ended is refilled from the warp's chunk (ballot + popc ranks the
 // idle lanes) as soon as a quarter of the warp is idle, so long and short
 // rays share warps. Ray state stays in registers for the whole ray.
 // Per-request counters are aggregated across the lanes of a warp that finish
-// together (match_any + reduce) before one atomic per request. Rays over their drift budget after passing inside
-// r = 4 are queued for an FP64 re-integration kernel that runs after the
-// wave. The wave (counter reset, persistent kernel, FP64 pass) is captured
-// once per slot into a CUDA graph and replayed; only the wave's descriptors
-// are copied in before each replay.
+// together (match_any + reduce) before one atomic per request. Rays over
+// their drift budget after passing inside r = 4 are queued for an FP64
+// re-integration kernel that runs after the wave, on a stream of its own. The
+// wave's two kernels are captured once per slot into a CUDA graph and
+// replayed (choose_kerr_kernel sets the Kerr kernel where it changes); only
+// the wave's descriptors are copied in before each replay.
 //
 // Host side. A scheduler thread admits submitted requests in arrival order
 // while their device footprint fits the server's memory (the HBM admission
@@ -240,8 +240,8 @@ __device__ void serve_queue(const WaveArgs& a, uint32_t lane) {
                         r = s_finish(L, R.u, t, a.blackbody);
                     }
                 } else {
-                    const LaneView v{R.u.geodesic.stepFactor, R.u.geodesic.escapeRadius, a.minus_zero, R.emission != 0, &R.u, R.emission,
-                                     R.velocity};
+                    const LaneView v{R.u.geodesic.stepFactor, R.u.geodesic.escapeRadius, a.minus_zero,
+                                     R.emission != 0, &R.u, R.emission, R.velocity};
                     kerr_step(L, v, taken);
                     if (++taken >= step_cap(R.u)) kerr_exhaust(L, taken);
                     finished = !any_alive(L.sh);
@@ -374,7 +374,8 @@ __device__ void serve_kerr_chunks(const WaveArgs& a, uint32_t lane, GatherWords*
         const ServeChunk ch = a.chunks1[c];
         const ServeRequest& q = a.requests[ch.request];
         __syncwarp();
-        if (lane == 0) *words = GatherWords{q.emission, q.velocity, q.u.volumeHalfExtent, q.u.opacityScale, q.u.redshift, 0u};
+        if (lane == 0)
+            *words = GatherWords{q.emission, q.velocity, q.u.volumeHalfExtent, q.u.opacityScale, q.u.redshift, 0u};
         __syncwarp();
         const WarpView view{q.u.geodesic.stepFactor, q.u.geodesic.escapeRadius, a.minus_zero, q.emission != 0, words};
         kerr_chunk<R>(a, ch, q, view, lane);
@@ -772,8 +773,10 @@ static bool form_wave(gg_server* s, WaveSlot& w) {
     // more than the pairs save. Lone stills, one ray to a lane against pairs:
     // 230k rays 1180 us, 1280 (256 steps) and 2110, 2430 (4096); 360k 1515,
     // 1400 and 2240, 2410; 518k 2050, 1745 and 2680, 2660; 682k 2406, 2190
-    // and 3150, 2910. The line is at 3 rounds, 455k rays; the second part of
-    // two waves stays in pairs if the first was.
+    // and 3150, 2910. The line is at 3 rounds, 455k rays, where 4096-step
+    // requests break even. It looks at rays alone: 256-step requests break
+    // even near 300k, and between the two they take the slower kernel, by up
+    // to 8 %. The second part of two waves stays in pairs if the first was.
     uint64_t kerr_rays = 0;
     for (auto& r : cands)
         if (r->u.spin > 0.0f) kerr_rays += r->rays - r->next_ray;
@@ -785,7 +788,8 @@ static bool form_wave(gg_server* s, WaveSlot& w) {
     s->kerr_single = s->cfg.schedule == GG_SCHEDULE_CHUNKS && !(second && !s->kerr_single) &&
                      kerr_rays < 3ull * 64u * (uint64_t)s->grid_k * (kServeThreads / 32);
     w.kerr_single = s->kerr_single;
-    const uint32_t chunks_of[2] = {s->cfg.chunk_rays, w.kerr_single ? s->cfg.chunk_rays : std::max(64u, s->cfg.chunk_rays)};
+    const uint32_t chunks_of[2] = {s->cfg.chunk_rays,
+                                   w.kerr_single ? s->cfg.chunk_rays : std::max(64u, s->cfg.chunk_rays)};
     // Kerr rays that would make one last wave, with nothing else under way,
     // make two: the rays flagged for FP64 pass close to the hole, so they are
     // among the first two fifths (ray_pixel), and that part's FP64 pass, a
