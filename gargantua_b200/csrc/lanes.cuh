@@ -433,8 +433,8 @@ __device__ __forceinline__ bool s_step(SLane<R>& l, const MarchUniforms& u, cuda
     return false;
 }
 
-// The radius below which no step of a ray reaches the sphere: |rDot| is at
-// most E < 1. Infinite without the sphere.
+// The radius below which no step of a ray reaches the sphere as long as its
+// state is accurate: |rDot| is at most E < 1. Infinite without the sphere.
 __device__ __forceinline__ float s_inner(const MarchUniforms& u) {
     const float longest = fmaxf(u.geodesic.stepMax, u.geodesic.emptyStepMax);
     return u.sphereRadius > 0.0f ? fmaf(-1.05f, longest, u.sphereRadius) : INFINITY;
